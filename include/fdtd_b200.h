@@ -78,8 +78,9 @@ typedef struct {
  * staggers (cpml.py:111-134, engine.py:264-283), and the 12 ψ stripes.
  * psi_h order: Hx_y, Hx_z, Hy_x, Hy_z, Hz_x, Hz_y;
  * psi_e order: Ex_y, Ex_z, Ey_x, Ey_z, Ez_x, Ez_y (yee_update.cl:56-58,176-178).
- * Every entry point updates the ψ stripes in place; psi_h_next is reserved
- * (ignored, may be NULL). */
+ * The ψ stripes are updated in place, except that fdtd_step_swap writes the
+ * advanced ψ_H to psi_h_next; every other entry point ignores psi_h_next (it
+ * may be NULL). */
 typedef struct {
     const void *b_h[3], *c_h[3], *ik_h[3];
     const void *b_e[3], *c_e[3], *ik_e[3];
@@ -140,6 +141,18 @@ int fdtd_update_E(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
 int fdtd_step(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
               const fdtd_source *src, int32_t nsrc,
               const fdtd_plane_dft *planes, int32_t nplanes, void *stream);
+
+/* The same step with ψ_H double-buffered like the fields: psi_h is read and
+ * every advanced ψ_H value written to psi_h_next (all six set, none aliasing
+ * psi_h; may be NULL when npml == 0), and the caller swaps the two sets along
+ * with E/E_next and H/H_next; ψ_E in place.  With ψ_H kept, a CTA can evaluate
+ * H^{n+1/2} of a neighbour's CPML cell, so whole grids whose step exceeds the L2
+ * (two million FP32 cells and more, rows a multiple of 16 bytes) take one march
+ * over all cells instead of fdtd_step's interior and shell launches.  Same
+ * results bit for bit. */
+int fdtd_step_swap(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
+                   const fdtd_source *src, int32_t nsrc,
+                   const fdtd_plane_dft *planes, int32_t nplanes, void *stream);
 
 /* Immediate sheet injection into Ex (used when a source callback reads fields
  * after injecting).  Replaces add_source_Jx / add_source_Ex
@@ -369,7 +382,8 @@ int fdtd_set_epsilon(const fdtd_grid *g, const void *eps, const void *sigma, int
  * DFT (of the interior cells, or with the face marches of the whole planes),
  * [4] the shell E cells after the join (the face marches and the per-cell
  * edges beside them, or the per-cell kernel with sources and DFTs), and the
- * number of steps recorded.  No reference counterpart. */
+ * number of steps recorded.  A step that runs as one march (fdtd_step_swap) has
+ * it in [2]; [0], [1] and [4] are then empty.  No reference counterpart. */
 int fdtd_profile_steps(int32_t enable);
 int fdtd_profile_read(double ms[5], int32_t *nsteps);
 

@@ -106,6 +106,8 @@ SIGNATURES = {
                                 c_int32, POINTER(PlaneDft), c_int32, c_void_p]),
     "fdtd_step": (c_int32, [POINTER(Grid), POINTER(Fields), POINTER(Cpml), POINTER(Source),
                             c_int32, POINTER(PlaneDft), c_int32, c_void_p]),
+    "fdtd_step_swap": (c_int32, [POINTER(Grid), POINTER(Fields), POINTER(Cpml), POINTER(Source),
+                                 c_int32, POINTER(PlaneDft), c_int32, c_void_p]),
     "fdtd_add_source": (c_int32, [POINTER(Grid), c_void_p, c_void_p, POINTER(Source), c_void_p]),
     "fdtd_dft_faces": (c_int32, [POINTER(Grid), POINTER(c_void_p), POINTER(c_void_p),
                                  POINTER(Box), c_void_p, c_void_p, c_void_p]),

@@ -187,7 +187,8 @@ int build_planes(const fdtd_grid *g, const fdtd_plane_dft *pl, int np, fdtd::Pla
 }
 
 template <typename T>
-fdtd::YeeArgs<T> make_args(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c) {
+fdtd::YeeArgs<T> make_args(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
+                           bool swap = false) {
     fdtd::YeeArgs<T> a;
     memset(&a, 0, sizeof(a));
     a.nx = g->nx;
@@ -217,7 +218,7 @@ fdtd::YeeArgs<T> make_args(const fdtd_grid *g, const fdtd_fields *f, const fdtd_
     }
     for (int q = 0; q < 6; ++q) {
         a.psi_h[q] = (T *)c->psi_h[q];
-        a.psi_h_next[q] = (T *)c->psi_h_next[q];
+        a.psi_h_next[q] = (T *)(swap ? c->psi_h_next[q] : c->psi_h[q]);
         a.psi_e[q] = (T *)c->psi_e[q];
     }
     return a;
@@ -472,22 +473,38 @@ int fdtd_update_E(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
                        "update_E");
 }
 
-int fdtd_step(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
-              const fdtd_source *src, int32_t nsrc, const fdtd_plane_dft *planes,
-              int32_t nplanes, void *stream) {
+static int step_impl(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
+                     const fdtd_source *src, int32_t nsrc, const fdtd_plane_dft *planes,
+                     int32_t nplanes, void *stream, bool swap, const char *what) {
     int rc;
     if ((rc = check_grid(g)) || (rc = check_fields(g, f, true)) || (rc = check_cpml(g, c)))
         return rc;
+    if (swap && g->npml > 0)
+        for (int q = 0; q < 6; ++q)
+            if (!c->psi_h_next[q] || c->psi_h_next[q] == c->psi_h[q])
+                return fail(FDTD_ERR_INVALID, "psi_h_next[%d] is NULL or aliases psi_h", q);
     fdtd::SourceList sl;
     fdtd::PlaneList pl;
     if ((rc = build_sources(g, src, nsrc, sl)) || (rc = build_planes(g, planes, nplanes, pl)))
         return rc;
     cudaStream_t st = (cudaStream_t)stream;
     if (g->dtype == FDTD_F32)
-        return cuda_status(fdtd::launch_step_fused<float>(make_args<float>(g, f, c), sl, pl, st),
-                           "step");
-    return cuda_status(fdtd::launch_step_fused<double>(make_args<double>(g, f, c), sl, pl, st),
-                       "step");
+        return cuda_status(
+            fdtd::launch_step_fused<float>(make_args<float>(g, f, c, swap), sl, pl, st), what);
+    return cuda_status(
+        fdtd::launch_step_fused<double>(make_args<double>(g, f, c, swap), sl, pl, st), what);
+}
+
+int fdtd_step(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
+              const fdtd_source *src, int32_t nsrc, const fdtd_plane_dft *planes,
+              int32_t nplanes, void *stream) {
+    return step_impl(g, f, c, src, nsrc, planes, nplanes, stream, false, "step");
+}
+
+int fdtd_step_swap(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
+                   const fdtd_source *src, int32_t nsrc, const fdtd_plane_dft *planes,
+                   int32_t nplanes, void *stream) {
+    return step_impl(g, f, c, src, nsrc, planes, nplanes, stream, true, "step_swap");
 }
 
 int fdtd_add_source(const fdtd_grid *g, void *Ex, const void *ce_x, const fdtd_source *src,

@@ -543,13 +543,13 @@ void set_chunks(FaceBox &f, int nplanes) {
 // E cells.
 constexpr int64_t FACE_MIN_CELLS = 20000000;
 
+}  // namespace
+
 int face_mode() {
     const char *e = getenv("FDTD_B200_FACE_E");
     if (!e || !*e) return -1;
     return atoi(e) != 0 ? 1 : 0;
 }
-
-}  // namespace
 
 // The six CPML face regions and the box list of the remaining shell E cells
 // (P = npml, I = [P+1, N-P)): the x edges of the planes [0, P] and [N-P, N)

@@ -1,6 +1,8 @@
 // Fused Yee step for sm_100a: one pass over HBM for the interior of the grid.
 //
-// Schedule of fdtd_step (two streams):
+// Schedules: a whole grid stepped with ψ_H double-buffered (fdtd_step_swap) and
+// too large for the L2 takes one march over every cell (yee_march.cu).  The
+// others (ψ_H in place, x-slabs, odd rows, small grids) run, on two streams:
 //   side stream, forked from the caller's stream:
 //   1. k_shell_H   (yee_shell.cu): H^{n+1/2} on the CPML shell outside the box
 //                  B = [npml, N-npml)^3, psi_H in place, into H_next.
@@ -62,6 +64,7 @@
 #include <unordered_map>
 
 #include "launch_count.cuh"
+#include "shell_plan.cuh"
 #include "tma.cuh"
 #include "yee_launch.cuh"
 
@@ -758,11 +761,40 @@ bool split_shell_e() {
     return v;
 }
 
+// The step as one march over the whole grid, then the monitored planes' DFTs.
+template <typename T>
+static cudaError_t launch_step_march(const YeeArgs<T> &a, const SourceList &src,
+                                     const PlaneList &pl, cudaStream_t st) {
+    std::array<cudaEvent_t, NEV> ev;
+    const bool prof = prof_begin(ev);
+    if (prof)
+        for (int s = 0; s < 3; ++s) cudaEventRecord(ev[s], st);
+    cudaError_t e = launch_march<T>(a, src, st);
+    if (e == cudaErrorNotSupported) {
+        if (prof)
+            for (cudaEvent_t x : ev) cudaEventDestroy(x);
+        return e;
+    }
+    if (prof)
+        for (int s = 3; s < 6; ++s) cudaEventRecord(ev[s], st);
+    const ShellBox all = whole_grid(a.nx, a.ny, a.nz);
+    if (e == cudaSuccess && pl.n) e = launch_plane_dft_box<T>(a, all, pl, st);
+    if (prof) {
+        cudaEventRecord(ev[6], st);
+        prof_end(ev, true);
+    }
+    return e;
+}
+
 template <typename T>
 cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const PlaneList &pl,
                               cudaStream_t st) {
     const int elem = (int)sizeof(T);
     const int n[3] = {a.nx, a.ny, a.nz};
+    if (face_mode() != 1 && march_path_ok<T>(a)) {
+        const cudaError_t e = launch_step_march<T>(a, src, pl, st);
+        if (e != cudaErrorNotSupported) return e;  // else no tensor maps, nothing launched
+    }
     // interior H box B = [npml, N-npml)^3 (x on a slab: [pml_lo, nx - pml_hi -
     // ghost_hi), so the upper ghost plane, whose forward differences would read
     // past the slab, is left to the boundary-guarded shell kernel); the fused
@@ -892,9 +924,9 @@ void set_interior_wait_polls(int64_t polls) {
                                  : (long long)(polls > (int64_t)WAIT_LIMIT ? WAIT_LIMIT : polls));
 }
 
-// The interior kernel's and the face kernels' flags (one status bit).
+// The plane-marching kernels' flags (one status bit).
 int read_fused_error(int reset) {
-    const int f = read_face_error(reset);
+    const int f = read_face_error(reset) | read_march_error(reset);
     int v = 0;
     cudaMemcpyFromSymbol(&v, g_fused_error, sizeof(int));
     if (reset) {

@@ -8,7 +8,8 @@ namespace fdtd {
 
 // Everything a Yee kernel needs, by value (device pointers + scalars already
 // rounded to T).  E/H are read (and, for the split kernels, written in place);
-// E_next/H_next/psi_h_next are the fused kernel's outputs.
+// E_next/H_next are the fused step's outputs, psi_h_next its advanced psi_H
+// (== psi_h: in place).
 template <typename T>
 struct YeeArgs {
     int nx, ny, nz, npml, lossy;
@@ -57,12 +58,22 @@ struct SideStream;
 // with nothing launched, when the tensor maps cannot be built.  face_path_ok:
 // the grid qualifies (whole grid, npml a multiple of 16 bytes of elements,
 // aligned stripes).
+int face_mode();  // FDTD_B200_FACE_E: 1 forced on, 0 off, -1 unset
 template <typename T>
 bool face_path_ok(const YeeArgs<T> &a);
 template <typename T>
 cudaError_t launch_shell_E_faces(const YeeArgs<T> &a, const SourceList &src, cudaStream_t st,
                                  SideStream *side);
 int read_face_error(int reset);
+
+// The whole step but the plane DFTs as one plane march over the grid, CPML
+// included (yee_march.cu): reads E/H/psi_h, writes E_next/H_next/psi_h_next,
+// psi_e in place.  march_path_ok: the grid and buffers qualify.
+template <typename T>
+bool march_path_ok(const YeeArgs<T> &a);
+template <typename T>
+cudaError_t launch_march(const YeeArgs<T> &a, const SourceList &src, cudaStream_t st);
+int read_march_error(int reset);
 unsigned interior_wait_polls();
 
 template <typename T>

@@ -5,7 +5,8 @@
 // thread per cell:
 //   k_shell_H : H^{n+1/2} of every cell outside the box B = [lo, hi)^3 (the
 //               CPML slabs; the whole grid when there is no box), H read from H
-//               and written to H_next, psi_H in place.
+//               and written to H_next, psi_H into psi_h_next (the same stripes
+//               or, in the swapping step, the next set).
 //   k_shell_E : E^{n+1} of the cells of an outer box that lie outside an inner
 //               box, reading H^{n+1/2} from H_next, writing E_next, psi_E in
 //               place, with the sheet injections and plane DFTs of those cells.
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(SHELL_THREADS)
     d.xy = (j < ny - 1) ? (Ex[idx + sy] - ex0) : T(0);
     T hx = a.H[0][idx], hy = a.H[1][idx], hz = a.H[2][idx];
     h_cell<T, true>(interior, i, j, k, nx, ny, nz, npml, a.xb, a.dtm, a.dtm_dl, d, a.cph, a.psi_h,
-                    a.psi_h, hx, hy, hz);
+                    a.psi_h_next, hx, hy, hz);
     a.H_next[0][idx] = hx;
     a.H_next[1][idx] = hy;
     a.H_next[2][idx] = hz;

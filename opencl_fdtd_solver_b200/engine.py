@@ -11,8 +11,8 @@ Reference contract (``opencl_fdtd_solver/engine.py``):
   monitor needs (``fdtd_read_regions``)
 
 Design.  Torch tensors own every device buffer; the kernels are reached only
-through the C ABI of ``libfdtd_b200.so`` (``_capi.py``).  A step normally runs as
-one fused kernel (``fdtd_step``): source callbacks are executed *before* the
+through the C ABI of ``libfdtd_b200.so`` (``_capi.py``).  A step normally runs
+fused (``fdtd_step_swap``, fields and ψ_H double-buffered): source callbacks are executed *before* the
 launch, with ``t`` at the half step, and their ``add_source_*`` calls are
 recorded and applied in the kernel to ``E^n`` ahead of the E update, which is
 exactly the reference ordering (H^{n+½} never depends on the injection).  If a
@@ -250,6 +250,14 @@ class CUDAFDTD(SourceMonitorMixin):
         with torch.cuda.stream(self.queue):
             self._psi_h = [mk(s) for s in order]
             self._psi_e = [mk(s) for s in order]
+            # the fused step's second ψ_H set (``fdtd_step_swap``); a grid that fills
+            # the device does without it and steps through ``fdtd_step``
+            self._psi_hn = None
+            if self._fused_enabled and n > 0:
+                try:
+                    self._psi_hn = [mk(s) for s in order]
+                except torch.OutOfMemoryError:
+                    log.info("no memory for a second psi_H set; stepping with psi_H in place")
 
     def _build_structs(self):
         g = capi.Grid()
@@ -277,18 +285,20 @@ class CUDAFDTD(SourceMonitorMixin):
     def _refresh_structs(self):
         self._fields_by_parity = {}
         self._build_fields()
-        cp = capi.Cpml.from_buffer_copy(self._cpml_base)
-        for q in range(6):
-            cp.psi_h[q] = self._psi_h[q].data_ptr()
-            cp.psi_e[q] = self._psi_e[q].data_ptr()
-        self._cpml = cp
         self._grid.lossy = 1 if self.lossy else 0
 
     def _build_fields(self):
         cached = self._fields_by_parity.get(self._parity)
         if cached is not None:
-            self._fields = cached
+            self._fields, self._cpml = cached
             return
+        cp = capi.Cpml.from_buffer_copy(self._cpml_base)
+        for q in range(6):
+            cp.psi_h[q] = self._psi_h[q].data_ptr()
+            cp.psi_e[q] = self._psi_e[q].data_ptr()
+            if self._psi_hn is not None:
+                cp.psi_h_next[q] = self._psi_hn[q].data_ptr()
+        self._cpml = cp
         f = capi.Fields()
         for a in range(3):
             f.E[a] = self._E[a].data_ptr()
@@ -300,7 +310,7 @@ class CUDAFDTD(SourceMonitorMixin):
                 f.E_next[a] = self._En[a].data_ptr()
                 f.H_next[a] = self._Hn[a].data_ptr()
         self._fields = f
-        self._fields_by_parity[self._parity] = f
+        self._fields_by_parity[self._parity] = f, cp
 
     # -------------------------------------------------------------- materials
     def set_epsilon(self, eps_array, sigma_array=None):
@@ -442,7 +452,8 @@ class CUDAFDTD(SourceMonitorMixin):
         else:
             done = False
             if self._fused_enabled:
-                rc = capi.call("fdtd_step", self._grid, self._fields, self._cpml, sa, len(pend),
+                name = "fdtd_step" if self._psi_hn is None else "fdtd_step_swap"
+                rc = capi.call(name, self._grid, self._fields, self._cpml, sa, len(pend),
                                pd, len(planes), st)
                 if rc == capi.FDTD_OK:
                     self._swap()
@@ -450,7 +461,7 @@ class CUDAFDTD(SourceMonitorMixin):
                 elif rc == capi.FDTD_ERR_UNSUPPORTED:
                     self._fused_enabled = False
                 else:
-                    capi.check(rc, "fdtd_step")
+                    capi.check(rc, name)
             if not done:
                 capi.run("fdtd_update_H", self._grid, self._fields, self._cpml, st)
                 capi.run("fdtd_update_E", self._grid, self._fields, self._cpml, sa, len(pend), pd,
@@ -468,6 +479,8 @@ class CUDAFDTD(SourceMonitorMixin):
     def _swap(self):
         self._E, self._En = self._En, self._E
         self._H, self._Hn = self._Hn, self._H
+        if self._psi_hn is not None:
+            self._psi_h, self._psi_hn = self._psi_hn, self._psi_h
         self._parity ^= 1
         self._build_fields()
 
