@@ -53,7 +53,7 @@ constexpr int MARCH_MAX_PLANES = 64;  // planes of a chunk (x profiles kept in s
 constexpr unsigned MARCH_DRAIN_LIMIT = 1u << 20;
 
 struct alignas(64) MarchMaps {
-    CUtensorMap E[3], H[3], C[6];  // C: ce, then ca when lossy
+    CUtensorMap m[12];  // E, H, ce, then ca when lossy
 };
 
 // Tile columns (rows) 0 .. lo-1 and n-hi .. n-1 along k (j) touch a z (y) slab.
@@ -164,22 +164,29 @@ __device__ __forceinline__ void march_tile(const MarchMaps &maps, const YeeArgs<
     }
     __syncthreads();
 
-    int last_issued = pfirst - 1;  // thread 0 only
-    auto issue = [&](int p) {      // plane p; E only for plane i1
+    // The warp after the cell threads, idle in the E phase, issues the copies of a
+    // plane (E only for plane i1): lane c copies array c, so the boxes' addresses
+    // are formed side by side.  (One cell thread issuing them all held its warp, and
+    // with it the CTA's next barrier, for several hundred cycles a plane.)
+    const int hl = tid - L::CELLTHR;
+    const int il = hl < 3 ? 0 : (hl < 6 ? 1 : 2);  // lane's array: E, H or coefficient
+    const int ioff = il == 0 ? hl * L::EB
+                             : (il == 1 ? 3 * L::EB + (hl - 3) * L::HB
+                                        : 3 * (L::EB + L::HB) + (hl - 6) * L::CB);
+    const int ik = il == 2 ? k0 : k0 - V, ij = il == 2 ? j0 : j0 - 1;
+    int last_issued = pfirst - 1;
+    auto issue = [&](int p) {  // by the whole warp
         const int s = (p - pfirst) % NSTAGE;
         last_issued = p;
-        unsigned char *st = smem + s * L::STAGE;
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(&bar[s], L::TX_E + (p < i1 ? L::TX_REST : 0u));
-        for (int c = 0; c < 3; ++c)
-            tma_load_3d(st + c * L::EB, &maps.E[c], &bar[s], k0 - V, j0 - 1, p);
-        if (p >= i1) return;
-        for (int c = 0; c < 3; ++c)
-            tma_load_3d(st + 3 * L::EB + c * L::HB, &maps.H[c], &bar[s], k0 - V, j0 - 1, p);
-        for (int c = 0; c < L::NCO; ++c)
-            tma_load_3d(st + 3 * (L::EB + L::HB) + c * L::CB, &maps.C[c], &bar[s], k0, j0, p);
+        if (hl == 0) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_expect_tx(&bar[s], L::TX_E + (p < i1 ? L::TX_REST : 0u));
+        }
+        __syncwarp();
+        if (hl < (p < i1 ? 6 + L::NCO : 3))
+            tma_load_3d(smem + s * L::STAGE + ioff, &maps.m[hl], &bar[s], ik, ij, p);
     };
-    if (tid == 0)
+    if (hl >= 0)
         for (int p = pfirst; p <= i1 && p < pfirst + NSTAGE; ++p) issue(p);
     // a zero budget gives up here, before the first plane can have landed
     bool w = bx.wait_polls != 0 || march_wait(&bar[0], 0, 0);
@@ -187,7 +194,6 @@ __device__ __forceinline__ void march_tile(const MarchMaps &maps, const YeeArgs<
     // this thread's vector: row r, group g of the tile; the warp after the cell
     // threads takes row -1 (lanes 0 .. G-1) and group -1 (lanes G .. G+TJ-1)
     const bool own = tid < L::CELLTHR;
-    const int hl = tid - L::CELLTHR;
     const int r = own ? tid / G : (hl < G ? -1 : (hl < G + TJ ? hl - G : 0));
     const int g = own ? tid % G : (hl < G ? hl : -1);
     const int j = j0 + r, kb = k0 + V * g;
@@ -470,7 +476,7 @@ __device__ __forceinline__ void march_tile(const MarchMaps &maps, const YeeArgs<
             ok = false;
             break;
         }
-        if (tid == 0 && p > pfirst && p - 1 + NSTAGE <= i1) issue(p - 1 + NSTAGE);
+        if (hl >= 0 && p > pfirst && p - 1 + NSTAGE <= i1) issue(p - 1 + NSTAGE);
         if (own && main) {
             T hzj[V], hxj[V], hxk[V], hyk[V], cex[V], cey[V], cez[V], cax[V], cay[V], caz[V];
             ld_vec<T, V>(nh + 2 * NE - HW, hzj);
@@ -611,7 +617,7 @@ __device__ __forceinline__ void march_tile(const MarchMaps &maps, const YeeArgs<
         // drain: every copy issued must land before the CTA exits; only the
         // last NSTAGE issued planes can still be in flight
         __syncthreads();
-        if (tid == 0) {
+        if (hl == 0) {
             const int from = max(pfirst, last_issued - NSTAGE + 1);
             for (int p = from; p <= last_issued; ++p) {
                 const int s = (p - pfirst) % NSTAGE;
@@ -757,11 +763,12 @@ bool build_march_maps(const YeeArgs<T> &a, MarchMaps &m) {
     if (cache.get(key, m)) return true;
     memset(&m, 0, sizeof(m));
     for (int c = 0; c < 3; ++c)
-        if (!make_tensor_map(&m.E[c], a.E[c], a.nx, a.ny, a.nz, elem, L::EW, L::EH) ||
-            !make_tensor_map(&m.H[c], a.H[c], a.nx, a.ny, a.nz, elem, L::HW, L::HH))
+        if (!make_tensor_map(&m.m[c], a.E[c], a.nx, a.ny, a.nz, elem, L::EW, L::EH) ||
+            !make_tensor_map(&m.m[3 + c], a.H[c], a.nx, a.ny, a.nz, elem, L::HW, L::HH))
             return false;
     for (int c = 0; c < L::NCO; ++c)
-        if (!make_tensor_map(&m.C[c], coef[c], a.nx, a.ny, a.nz, elem, L::TK, L::TJ)) return false;
+        if (!make_tensor_map(&m.m[6 + c], coef[c], a.nx, a.ny, a.nz, elem, L::TK, L::TJ))
+            return false;
     cache.put(key, m);
     return true;
 }
