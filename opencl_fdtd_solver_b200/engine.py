@@ -245,17 +245,24 @@ class CUDAFDTD(SourceMonitorMixin):
             sx = sy = sz = (1,)
         if sx[0] == 0:
             sx = (1,)  # a slab without x-CPML faces: the stripe is never indexed
-        mk = lambda s: torch.zeros(s, dtype=self._tdt, device=self.device)  # noqa: E731
         order = (sy, sz, sx, sz, sx, sy)  # Hx_y, Hx_z, Hy_x, Hy_z, Hz_x, Hz_y / E likewise
+        # one zeroed buffer a set, stripes on 256-byte boundaries
+        pitch = [-(-int(np.prod(s)) // 64) * 64 for s in order]
+
+        def stripes():
+            buf = torch.zeros(sum(pitch), dtype=self._tdt, device=self.device)
+            return [buf[o:o + int(np.prod(s))].view(s)
+                    for s, o in zip(order, np.cumsum([0] + pitch[:-1]).tolist())]
+
         with torch.cuda.stream(self.queue):
-            self._psi_h = [mk(s) for s in order]
-            self._psi_e = [mk(s) for s in order]
+            self._psi_h = stripes()
+            self._psi_e = stripes()
             # the fused step's second ψ_H set (``fdtd_step_swap``); a grid that fills
             # the device does without it and steps through ``fdtd_step``
             self._psi_hn = None
             if self._fused_enabled and n > 0:
                 try:
-                    self._psi_hn = [mk(s) for s in order]
+                    self._psi_hn = stripes()
                 except torch.OutOfMemoryError:
                     log.info("no memory for a second psi_H set; stepping with psi_H in place")
 
