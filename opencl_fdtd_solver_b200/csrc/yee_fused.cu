@@ -786,6 +786,38 @@ static cudaError_t launch_step_march(const YeeArgs<T> &a, const SourceList &src,
     return e;
 }
 
+// The step as two launches over the whole grid, one thread per cell (yee_shell.cu
+// with an empty inner box), plane DFTs fused.
+template <typename T>
+static cudaError_t launch_step_grid(const YeeArgs<T> &a, const SourceList &src,
+                                    const PlaneList &pl, cudaStream_t st) {
+    std::array<cudaEvent_t, NEV> ev;
+    const bool prof = prof_begin(ev);
+    if (prof) cudaEventRecord(ev[0], st);
+    ShellBox none;
+    memset(&none, 0, sizeof(none));
+    cudaError_t e = launch_shell_H<T>(a, none, st);
+    if (prof)
+        for (int s = 1; s < 6; ++s) cudaEventRecord(ev[s], st);
+    if (e == cudaSuccess) e = launch_shell_E<T>(a, none, src, pl, st);
+    if (prof) {
+        cudaEventRecord(ev[6], st);
+        prof_end(ev, false);
+    }
+    return e;
+}
+
+// Grids of this many cells that no march takes run as the two whole-grid
+// launches where these beat the interior march with shell kernels: small grids,
+// lossy ones with much CPML, and those whose z slabs (short rows for the shell
+// kernels) hold two fifths of the grid.  Measured per step, two launches / interior march, in us: FP32 with
+// a source and a plane DFT 48³ 13.5 / 24.7, 64³ 16.4 / 25.3, 96³ 28.0 / 31.4, 128³
+// 59.7 / 60.5; without, 46x445x288 npml 10 lossy 142.3 / 145.8, 300x300x60 npml 20
+// 133.0 / 163.8, 34x483x224 npml 13 96.1 / 96.3, 64x376x144 npml 16 88.3 / 84.9.
+// The two launches win below the line too (40x36x48 14.3 / 27.3), but the bounded
+// waits of the interior march and its launch counts are checked on such a grid.
+constexpr int64_t GRID_MIN_CELLS = 100000;
+
 template <typename T>
 cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const PlaneList &pl,
                               cudaStream_t st) {
@@ -795,6 +827,13 @@ cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const 
         const cudaError_t e = launch_step_march<T>(a, src, pl, st);
         if (e != cudaErrorNotSupported) return e;  // else no tensor maps, nothing launched
     }
+    const int64_t cells = (int64_t)a.nx * a.ny * a.nz;
+    if (face_mode() != 1 && cells >= GRID_MIN_CELLS &&
+        (!march_size<T>(cells) ||
+         (!a.ghost_lo && !a.ghost_hi &&
+          (5 * a.npml >= a.nz ||
+           (a.lossy && pml_fraction(a.nx, a.ny, a.nz, a.npml) >= 0.4)))))
+        return launch_step_grid<T>(a, src, pl, st);
     // interior H box B = [npml, N-npml)^3 (x on a slab: [pml_lo, nx - pml_hi -
     // ghost_hi), so the upper ghost plane, whose forward differences would read
     // past the slab, is left to the boundary-guarded shell kernel); the fused
@@ -829,57 +868,45 @@ cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const 
     FusedMaps maps;
     if (use_interior && !(gsel == 8 ? build_maps<T, 8>(a, maps) : build_maps<T, 16>(a, maps)))
         use_interior = false;
+    if (!use_interior) return launch_step_grid<T>(a, src, pl, st);
     // hbox = B (H of the interior kernel), ebox = B' (its E), rbox = [lo, hi+1):
     // the E cells outside rbox read no H of B, the rim rbox \ B' does
-    ShellBox hbox, ebox, rbox, none, all;
+    ShellBox hbox, ebox, rbox, all;
     for (int d = 0; d < 3; ++d) {
         all.lo[d] = 0;
         all.hi[d] = n[d];
-        hbox.lo[d] = use_interior ? blo[d] : 0;
-        hbox.hi[d] = use_interior ? bhi[d] : 0;
-        ebox.lo[d] = use_interior ? blo[d] + 1 : 0;
-        ebox.hi[d] = use_interior ? bhi[d] : 0;
-        rbox.lo[d] = use_interior ? blo[d] : 0;
-        rbox.hi[d] = use_interior ? bhi[d] + 1 : n[d];
-        none.lo[d] = none.hi[d] = 0;
+        hbox.lo[d] = blo[d];
+        hbox.hi[d] = bhi[d];
+        ebox.lo[d] = blo[d] + 1;
+        ebox.hi[d] = bhi[d];
+        rbox.lo[d] = blo[d];
+        rbox.hi[d] = bhi[d] + 1;
     }
     SideStream *side = nullptr;
-    if (use_interior) {
-        cudaError_t e = side_stream(&side);
-        if (e != cudaSuccess) return e;
-    }
+    cudaError_t e = side_stream(&side);
+    if (e != cudaSuccess) return e;
     std::array<cudaEvent_t, NEV> ev;
     const bool prof = prof_begin(ev);
     if (prof) cudaEventRecord(ev[0], st);
-    cudaError_t e = cudaSuccess;
-    if (use_interior) {
-        // shell H, then the outer shell E, on the side stream, concurrent with
-        // the interior kernel
-        if ((e = cudaEventRecord(side->fork, st)) == cudaSuccess &&
-            (e = cudaStreamWaitEvent(side->s, side->fork, 0)) == cudaSuccess)
-            e = launch_shell_H<T>(a, hbox, side->s);
-        if (prof) cudaEventRecord(ev[1], side->s);
-        if (e == cudaSuccess && split_shell_e())
-            e = launch_shell_E_region<T>(a, all, rbox, src, pl, side->s);
-        if (prof) cudaEventRecord(ev[2], side->s);
-        cudaError_t e2 = cudaEventRecord(side->join, side->s);
-        if (e == cudaSuccess) e = e2;
-        if (e == cudaSuccess)
-            e = gsel == 8 ? launch_interior<T, 8>(a, maps, hbox, src, st)
-                          : launch_interior<T, 16>(a, maps, hbox, src, st);
-        if (prof) cudaEventRecord(ev[3], st);
-        e2 = cudaStreamWaitEvent(st, side->join, 0);
-        if (e == cudaSuccess) e = e2;
-    } else {
-        e = launch_shell_H<T>(a, none, st);
-        if (prof) {
-            cudaEventRecord(ev[1], st);
-            cudaEventRecord(ev[2], st);
-            cudaEventRecord(ev[3], st);
-        }
-    }
+    // shell H, then the outer shell E, on the side stream, concurrent with the
+    // interior kernel
+    if ((e = cudaEventRecord(side->fork, st)) == cudaSuccess &&
+        (e = cudaStreamWaitEvent(side->s, side->fork, 0)) == cudaSuccess)
+        e = launch_shell_H<T>(a, hbox, side->s);
+    if (prof) cudaEventRecord(ev[1], side->s);
+    if (e == cudaSuccess && split_shell_e())
+        e = launch_shell_E_region<T>(a, all, rbox, src, pl, side->s);
+    if (prof) cudaEventRecord(ev[2], side->s);
+    cudaError_t e2 = cudaEventRecord(side->join, side->s);
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess)
+        e = gsel == 8 ? launch_interior<T, 8>(a, maps, hbox, src, st)
+                      : launch_interior<T, 16>(a, maps, hbox, src, st);
+    if (prof) cudaEventRecord(ev[3], st);
+    e2 = cudaStreamWaitEvent(st, side->join, 0);
+    if (e == cudaSuccess) e = e2;
     if (prof) cudaEventRecord(ev[4], st);
-    bool faces = use_interior && !split_shell_e() && face_path_ok<T>(a);
+    bool faces = !split_shell_e() && face_path_ok<T>(a);
     if (faces && e == cudaSuccess) {
         // shell E through the CPML face marches, then the plane DFTs of every
         // monitored cell in one pass over the planes
@@ -894,15 +921,12 @@ cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const 
         if (e == cudaSuccess && pl.n) e = launch_plane_dft_box<T>(a, all, pl, st);
     } else {
         // plane DFTs of the cells the interior kernel updated
-        if (e == cudaSuccess && use_interior && pl.n)
-            e = launch_plane_dft_box<T>(a, ebox, pl, st);
+        if (e == cudaSuccess && pl.n) e = launch_plane_dft_box<T>(a, ebox, pl, st);
         if (prof) cudaEventRecord(ev[5], st);
-        // E of the rim (or of the whole grid without an interior box), or of
-        // every cell outside B' when the outer part did not run on the side
-        // stream, with the DFTs of those cells
+        // E of the rim, or of every cell outside B' when the outer part did not
+        // run on the side stream, with the DFTs of those cells
         if (e == cudaSuccess)
-            e = launch_shell_E_region<T>(a, (use_interior && split_shell_e()) ? rbox : all, ebox,
-                                         src, pl, st);
+            e = launch_shell_E_region<T>(a, split_shell_e() ? rbox : all, ebox, src, pl, st);
     }
     if (prof) {
         cudaEventRecord(ev[6], st);

@@ -66,6 +66,37 @@ cudaError_t launch_shell_E_faces(const YeeArgs<T> &a, const SourceList &src, cud
                                  SideStream *side);
 int read_face_error(int reset);
 
+// Fraction of a grid's cells in a CPML slab.
+inline double pml_fraction(int nx, int ny, int nz, int npml) {
+    auto in = [&](int n) { return n > 2 * npml ? (double)(n - 2 * npml) / n : 0.0; };
+    return 1.0 - in(nx) * in(ny) * in(nz);
+}
+
+// The march takes grids whose step (15 arrays: six fields read, six written,
+// three coefficients) clearly exceeds the 126 MB L2.  Below, more threads beat
+// fewer bytes: the march's planes follow one another, about 1.7 us each.
+// Measured per step with a source and a plane DFT, march against one whole-grid H
+// and one E launch: FP32 64³ 20.6 / 16.4 us, 96³ 29.8 / 28.0, 128³ 64.4 / 59.7,
+// 160x160x96 69.1 / 69.8, 192³ 141.9 / 174.5; FP64 96³ 62.3 / 44.2, 128³ 85.5 / 95.9.
+constexpr int64_t MARCH_MIN_BYTES = 140000000;
+template <typename T>
+inline bool march_size(int64_t cells) {
+    return 15 * cells * (int64_t)sizeof(T) >= MARCH_MIN_BYTES;
+}
+
+// And whose CPML is not most of the grid: its CPML tiles evaluate their cells in
+// fewer, longer threads.  In ps per FP32 cell the march costs about (11 + 20 f)
+// per cell of its (padded) tiles, f the CPML fraction, 1.17 times that with ca; the
+// two whole-grid launches 21 + 4 f, 1.08 times with ca.  Measured, march / whole-grid
+// launches in us: 256³ npml 20 lossy (f 0.40) 349.9 / 363.9, 192³ npml 20 lossy
+// (0.50) 161 / 171, 100x300x200 npml 20 (0.58) 154.4 / 137.5, 160³ npml 20 lossy
+// (0.58) 124.2 / 108.6, 34x483x224 npml 13 (0.80) 117.8 / 94.6.
+inline bool march_pays(int nx, int ny, int nz, int npml, bool lossy, int tk, int tj) {
+    const double pad = (double)((nz + tk - 1) / tk * tk) / nz * ((ny + tj - 1) / tj * tj) / ny;
+    const double f = pml_fraction(nx, ny, nz, npml);
+    return pad * (11.0 + 20.0 * f) * (lossy ? 1.17 : 1.0) < (21.0 + 4.0 * f) * (lossy ? 1.08 : 1.0);
+}
+
 // The whole step but the plane DFTs as one plane march over the grid, CPML
 // included (yee_march.cu): reads E/H/psi_h, writes E_next/H_next/psi_h_next,
 // psi_e in place.  march_path_ok: the grid and buffers qualify.

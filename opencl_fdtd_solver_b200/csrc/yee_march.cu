@@ -825,13 +825,13 @@ cudaError_t launch_march_t(const YeeArgs<T> &a, const SourceList &src, cudaStrea
     return cudaGetLastError();
 }
 
-// The march takes grids whose step (15 arrays: six fields read, six written,
-// three coefficients) no longer fits the 126 MB L2.  Below, more threads beat
-// fewer bytes: the march's planes follow one another, about 1.7 us each.
-// Measured per step with a source and a plane DFT, march against one whole-grid H
-// and one E launch: FP32 64³ 20.6 / 16.4 us, 96³ 29.8 / 28.0, 128³ 64.4 / 59.7,
-// 160x160x96 69.1 / 69.8, 192³ 141.9 / 174.5; FP64 96³ 62.3 / 44.2, 128³ 85.5 / 95.9.
-constexpr int64_t MARCH_MIN_BYTES = 120000000;
+// 64 x 8 (FP64: 32 x 8) streams better; the narrower tile is taken where it saves
+// a fifth of the padded k extent.
+template <typename T>
+bool march_narrow(int nz) {
+    constexpr int W = 256 / (int)sizeof(T), N = W / 2;
+    return 5 * ((nz + W - 1) / W * W) > 6 * ((nz + N - 1) / N * N);
+}
 
 bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
@@ -855,16 +855,17 @@ bool march_path_ok(const YeeArgs<T> &a) {
         if (!aligned16(a.E[c]) || !aligned16(a.H[c]) || !aligned16(a.E_next[c]) ||
             !aligned16(a.H_next[c]) || !aligned16(a.ce[c]) || (a.lossy && !aligned16(a.ca[c])))
             return false;
-    return (int64_t)15 * a.nx * a.ny * a.nz * (int64_t)sizeof(T) >= MARCH_MIN_BYTES;
+    if (!march_size<T>((int64_t)a.nx * a.ny * a.nz)) return false;
+    const bool narrow = march_narrow<T>(a.nz);
+    const int tk = (narrow ? 128 : 256) / (int)sizeof(T), tj = narrow ? 16 : 8;
+    return march_pays(a.nx, a.ny, a.nz, P, a.lossy != 0, tk, tj);
 }
 
 // cudaErrorNotSupported, with nothing launched, when the tensor maps cannot be built.
 template <typename T>
 cudaError_t launch_march(const YeeArgs<T> &a, const SourceList &src, cudaStream_t st) {
-    // 64 x 8 (FP64: 32 x 8) streams better; the narrower tile is taken where it
-    // saves a fifth of the padded k extent
     constexpr int W = 256 / (int)sizeof(T), N = W / 2;
-    if (5 * ((a.nz + W - 1) / W * W) > 6 * ((a.nz + N - 1) / N * N))
+    if (march_narrow<T>(a.nz))
         return a.lossy ? launch_march_t<T, N, 16, true>(a, src, st)
                        : launch_march_t<T, N, 16, false>(a, src, st);
     return a.lossy ? launch_march_t<T, W, 8, true>(a, src, st)

@@ -3,7 +3,7 @@
 Grids above the size where ``fdtd_step_swap`` takes the march: extents that end
 inside a tile, slabs that end inside a vector (npml not a multiple of 16 bytes of
 elements) or a tile, one and several chunks along x, lossy media, sources and
-plane DFTs in the CPML; and one grid whose rows are no multiple of 16 bytes.
+plane DFTs in the CPML; and grids on the other side of each of its lines.
 """
 
 from __future__ import annotations
@@ -24,15 +24,17 @@ FIELDS = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
 
 CASES = [
     # shape, npml, lossy
-    ((200, 164, 64), 8, False),      # one tile along k
-    ((137, 153, 104), 5, True),      # partial tiles; vectors straddle the z slabs' edges
-    ((150, 166, 92), 6, False),      # straddling in FP32 only
-    ((570, 121, 36), 7, True),       # narrow tile, many planes: several chunks
-    ((26, 610, 132), 12, False),     # two planes between the x slabs; slab ends inside a j tile
-    ((244, 43, 200), 20, False),     # three planes between the y slabs
-    ((260, 210, 40), 18, False),     # four cells between the z slabs
-    ((1290, 41, 40), 1, False),      # one CPML layer
-    ((181, 142, 83), 9, True),       # odd rows: no march in FP32 and FP64
+    ((220, 170, 64), 4, False),      # one tile along k
+    ((137, 175, 104), 5, True),      # partial tiles; vectors straddle the z slabs' edges
+    ((150, 186, 92), 6, False),      # straddling in FP32 only
+    ((230, 131, 96), 3, True),       # narrow tile, many planes: several chunks
+    ((26, 680, 140), 2, False),      # few planes; slab ends inside a tile
+    ((244, 250, 64), 12, False),     # a rim row in the next tile
+    ((1000, 47, 60), 1, False),      # one CPML layer
+    ((181, 142, 103), 9, True),      # odd rows: two whole-grid launches
+    ((46, 445, 120), 16, True),      # mostly CPML, lossy: two whole-grid launches
+    ((90, 320, 84), 12, False),      # mostly CPML, lossless: interior march and shell kernels
+    ((70, 60, 56), 6, False),        # small: two whole-grid launches
 ]
 
 
@@ -86,7 +88,7 @@ def test_march_launches_and_wait_timeout():
         pytest.skip("no CUDA device")
     from opencl_fdtd_solver_b200 import CUDAFDTD, _capi as capi
 
-    g = CUDAFDTD((130, 130, 128), 1e-3, npml=8)
+    g = CUDAFDTD((160, 130, 128), 1e-3, npml=8)
     g.run(2)
     g.synchronize()
     n0 = capi.lib().fdtd_launch_count()
