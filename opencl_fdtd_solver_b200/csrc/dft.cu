@@ -8,7 +8,9 @@
 //                      monitors.py:560-569, as a deterministic two-pass reduce.
 //   k_farfield_nl    : dft_farfield.cl:372-556 (trapezoid weights, face-centre
 //                      sample positions, N = n x H, L = -n x E), one block per
-//                      observation point, block tree reduction (no atomics).
+//                      observation point, block tree reduction (no atomics);
+//                      k_farfield_nl_sep the same sums for many points, with
+//                      the phase separated per face and float64 mma.
 //   k_farfield_eh    : dft_farfield.cl:559-635 with the kernel's sign,
 //                      E = -jk e^{-jkr}/(4 pi r) (eta N_t - r x L), H = -r x E / eta.
 //
@@ -262,6 +264,201 @@ __global__ void __launch_bounds__(FF_THREADS)
     }
 }
 
+// The same sums with the phase separated over a face's rows and columns:
+//   e^{jk r̂·r'} = C(o) u_p(o) v_q(o),  u_p = e^{j2π γ_p p},  v_q = e^{j2π γ_q q},
+//   γ = k dl r̂ / 2π turns per sample,
+// so T[o][q][c] = Σ_p u_p cur[p][q][c] is a complex matrix product over the rows p
+// and NL += C Σ_q v_q T: four complex multiply-adds a sample and direction, in
+// place of a float64 sincos and its argument besides.  The products run as
+// float64 mma.sync m8n8k4 (full float64 multiply-adds): M = 8 directions, K = two
+// rows (Re, Im), N = one column's four currents (Re, Im), B = [[zr, zi], [-zi, zr]].
+// A lane's fragments: A(row lane/4, k lane%4), B(k lane%4, n lane/4), and in the
+// accumulator the complex T of direction lane/4, current lane%4.  A warp keeps
+// SEP_OBS directions x SEP_NT columns; columns are shared out over the block's warps.
+// u is rotated from row pair to row pair and evaluated afresh every SEP_ANCHOR
+// pairs, v likewise within a column group.
+//
+// Bound by the float64 pipe and by how evenly 16-direction blocks fill the SMs.
+// Float64 vector arithmetic has the same peak as float64 mma here (36 against 37
+// TFLOP/s measured), but a lane that keeps one direction issues a 16-byte load for
+// four multiply-adds, and the loads bind.  16471 directions x 47526 samples, the
+// whole call: 7.8 ms with k_farfield_nl, 3.3 to 4.7 ms with vector arithmetic, 1.7
+// ms with this kernel, of which 0.45 ms are the host's copies.  32 directions x 4
+// columns a warp take 1.9 ms, 16 x 4 at two blocks an SM 1.8.  The error against
+// float64 sums with phases in turns is not above that of k_farfield_nl, which
+// rounds k r̂·r' in radians.
+constexpr int SEP_WARPS = 8;
+constexpr int SEP_MT = 2, SEP_OBS = 8 * SEP_MT;
+constexpr int SEP_NT = 8;
+constexpr int SEP_ANCHOR = 32;
+
+// Turns per sample as an unevaluated sum of two doubles, and the fraction of n of
+// them: rounding the rate once would shift the phase of a whole face by the
+// rounding times its turns.
+struct Turns {
+    double h, l;
+};
+__device__ __forceinline__ Turns turn_rate(double k, double dl, double r) {
+    // k / 2π, then times dl r, the rounding of each product kept
+    const double ih = 0.15915494309189535, il = -9.839338337591243e-18;
+    const double kh = k * ih, kl = fma(k, ih, -kh) + k * il;
+    const double xh = dl * r, xl = fma(dl, r, -xh);
+    Turns t;
+    t.h = kh * xh;
+    t.l = fma(kh, xh, -t.h) + (kh * xl + kl * xh);
+    return t;
+}
+__device__ __forceinline__ double turn_frac(const Turns &g, double n) {
+    const double t = g.h * n;
+    return (t - rint(t)) + (fma(g.h, n, -t) + g.l * n);
+}
+__device__ __forceinline__ double2 turn_phase(double t) {
+    double s, c;
+    sincospi(2.0 * t, &s, &c);
+    return make_double2(c, s);
+}
+__device__ __forceinline__ double2 cmac(double2 a, double2 b, double2 acc) {
+    acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
+    acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
+    return acc;
+}
+__device__ __forceinline__ void mma_f64(double2 &d, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d.x), "+d"(d.y)
+        : "d"(a), "d"(b));
+}
+
+__global__ void __launch_bounds__(32 * SEP_WARPS)
+    k_farfield_nl_sep(fdtd_box b, const double *acc, int fi, double dl, double k_wave,
+                      const double *obs, int n_obs, double2 *nl) {
+    __shared__ double2 red[SEP_WARPS][6][SEP_OBS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t = lane; t < 6 * SEP_OBS; t += 32) (&red[warp][0][0])[t] = make_double2(0.0, 0.0);
+    __syncwarp();
+    // unit vectors of this lane's directions lane/4 + 8m
+    double rh[SEP_MT][3];
+#pragma unroll
+    for (int m = 0; m < SEP_MT; ++m) {
+        const int o = min(blockIdx.x * SEP_OBS + 8 * m + (lane >> 2), n_obs - 1);
+        const double ox = obs[3 * o], oy = obs[3 * o + 1], oz = obs[3 * o + 2];
+        double r = sqrt(ox * ox + oy * oy + oz * oz);
+        if (r < 1e-30) r = 1e-30;
+        rh[m][0] = ox / r;
+        rh[m][1] = oy / r;
+        rh[m][2] = oz / r;
+    }
+    const int lo[3] = {b.ix0, b.iy0, b.iz0}, hi[3] = {b.ix1, b.iy1, b.iz1};
+    const int64_t stride = 2 * (int64_t)b.nfreq * b.n_face;  // doubles of a component
+    const int kp = (lane >> 1) & 1, rk = lane & 1;           // row of the pair, Re / Im of u
+    const int cb = lane >> 3, rn = (lane >> 2) & 1;          // current, Re / Im of B's column
+    const bool neg = rk && !rn;
+    int item0 = 0;  // column groups of the faces before this one
+#pragma unroll 1
+    for (int face = 0; face < 6; ++face) {
+        const int n = face >> 1, ap = n == 0 ? 1 : 0, aq = n == 2 ? 1 : 2;
+        const int np = hi[ap] - lo[ap] + 1, nq = hi[aq] - lo[aq] + 1;
+        // currents in the order E_p, E_q, H_p, H_q
+        const int comp = cb == 0 ? ap : (cb == 1 ? aq : (cb == 2 ? 3 + ap : 3 + aq));
+        const double *src = acc + comp * stride +
+                            2 * ((int64_t)fi * b.n_face + b.off[face]) + (rk ^ rn);
+        const int groups = (nq + SEP_NT - 1) / SEP_NT;
+        const int g0 = (warp + SEP_WARPS - item0 % SEP_WARPS) % SEP_WARPS;
+        item0 += groups;
+        if (g0 >= groups) continue;
+        Turns gp[SEP_MT], gq[SEP_MT];
+        double2 W[SEP_MT], S[SEP_MT];
+#pragma unroll
+        for (int m = 0; m < SEP_MT; ++m) {
+            gp[m] = turn_rate(k_wave, dl, ap == 0 ? rh[m][0] : rh[m][1]);
+            gq[m] = turn_rate(k_wave, dl, aq == 1 ? rh[m][1] : rh[m][2]);
+            W[m] = turn_phase(turn_frac(gp[m], 2.0));
+            S[m] = make_double2(0.0, 0.0);
+        }
+        for (int g = g0; g < groups; g += SEP_WARPS) {
+            const int q0 = g * SEP_NT;
+            int at[SEP_NT];  // columns beyond the face repeat its last one, unused
+#pragma unroll
+            for (int t = 0; t < SEP_NT; ++t) at[t] = 2 * min(q0 + t, nq - 1);
+            double2 T[SEP_MT][SEP_NT];
+#pragma unroll
+            for (int m = 0; m < SEP_MT; ++m)
+#pragma unroll
+                for (int t = 0; t < SEP_NT; ++t) T[m][t] = make_double2(0.0, 0.0);
+            double z[SEP_NT];
+            {
+                const double *row = src + 2 * (int64_t)min(kp, np - 1) * nq;
+#pragma unroll
+                for (int t = 0; t < SEP_NT; ++t) z[t] = __ldg(row + at[t]);
+            }
+            double2 u[SEP_MT];
+            for (int p0 = 0; p0 < np; p0 += 2) {
+                const int p = p0 + kp;
+                double zn[SEP_NT];  // the next pair's samples, ahead of this pair's products
+                const double *row = src + 2 * (int64_t)min(p + 2, np - 1) * nq;
+#pragma unroll
+                for (int t = 0; t < SEP_NT; ++t) zn[t] = __ldg(row + at[t]);
+                const double w = p >= np ? 0.0 : ((p == 0 || p == np - 1) ? 0.5 : 1.0);
+                double A[SEP_MT];
+#pragma unroll
+                for (int m = 0; m < SEP_MT; ++m) {
+                    if (p0 % (2 * SEP_ANCHOR) == 0)
+                        u[m] = turn_phase(turn_frac(gp[m], p));
+                    else
+                        u[m] = cmac(u[m], W[m], make_double2(0.0, 0.0));
+                    A[m] = w * (rk ? u[m].y : u[m].x);
+                }
+#pragma unroll
+                for (int t = 0; t < SEP_NT; ++t) {
+                    const double B = neg ? -z[t] : z[t];
+#pragma unroll
+                    for (int m = 0; m < SEP_MT; ++m) mma_f64(T[m][t], A[m], B);
+                    z[t] = zn[t];
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < SEP_MT; ++m) {
+                double2 v = turn_phase(turn_frac(gq[m], q0));
+                const double2 Wq = turn_phase(turn_frac(gq[m], 1.0));
+#pragma unroll
+                for (int t = 0; t < SEP_NT; ++t) {
+                    const int q = q0 + t;
+                    if (q >= nq) break;
+                    const double w = (q == 0 || q == nq - 1) ? 0.5 : 1.0;
+                    S[m] = cmac(make_double2(v.x * w, v.y * w), T[m][t], S[m]);
+                    v = cmac(v, Wq, make_double2(0.0, 0.0));
+                }
+            }
+        }
+        // this lane's current lane%4 into its component of NL: N = -n x H and
+        // L = n x E of k_farfield_nl; (n, p, q) is cyclic for n = x, z, reversed for y
+        const int c = lane & 3;
+        const int dst = c == 0 ? 3 + aq : (c == 1 ? 3 + ap : (c == 2 ? aq : ap));
+        const double sg = ((face & 1) ? 1.0 : -1.0) * (n == 1 ? -1.0 : 1.0) *
+                          ((c == 1 || c == 2) ? -1.0 : 1.0) * (dl * dl);
+        const double xn = (face & 1) ? hi[n] : lo[n], yp = lo[ap] + 0.5, yq = lo[aq] + 0.5;
+#pragma unroll
+        for (int m = 0; m < SEP_MT; ++m) {
+            const Turns gn = turn_rate(k_wave, dl, n == 0 ? rh[m][0] : (n == 1 ? rh[m][1] : rh[m][2]));
+            const double2 C = turn_phase(turn_frac(gn, xn) + turn_frac(gp[m], yp) +
+                                         turn_frac(gq[m], yq));
+            double2 &s = red[warp][dst][8 * m + (lane >> 2)];
+            s = cmac(make_double2(C.x * sg, C.y * sg), S[m], s);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 6 * SEP_OBS; t += 32 * SEP_WARPS) {
+        const int c = t / SEP_OBS, l = t % SEP_OBS;
+        double2 v = make_double2(0.0, 0.0);
+        for (int w = 0; w < SEP_WARPS; ++w) {
+            v.x += red[w][c][l].x;
+            v.y += red[w][c][l].y;
+        }
+        const int dst = blockIdx.x * SEP_OBS + l;
+        if (dst < n_obs) nl[6 * (int64_t)dst + c] = v;
+    }
+}
+
 // NL may be complex128 (the direct sums) or complex64 (the tensor-core contraction).
 template <typename NT>
 __global__ void k_farfield_eh(const NT *nl, const double *obs, int n_obs, double k_wave,
@@ -405,12 +602,23 @@ cudaError_t launch_rel_change_noalloc(const double *cur, const double *prev, int
     return cudaGetLastError();
 }
 
+// A block of the separated sums takes its 16 directions through all samples, so
+// their time hardly falls below one wave of blocks; the direct sums, a block a
+// direction, win for few directions.  Whole calls, direct / separated, in us: 300
+// directions x 47526 samples 307 / 290, 73 x 47526 234 / 284, 500 x 6534 164 / 135,
+// 73 x 6534 110 / 123.
+constexpr int SEP_MIN_OBS = 400;
+
 cudaError_t launch_farfield(const fdtd_box &b, const double *acc, int fi, double dl,
                             double k_wave, double eta0, const double *obs, int n_obs,
                             double *nl, double *eh, cudaStream_t st) {
-    k_farfield_nl<<<n_obs, FF_THREADS, 0, st>>>(b, reinterpret_cast<const double2 *>(acc), fi,
-                                                dl, k_wave, obs, n_obs,
-                                                reinterpret_cast<double2 *>(nl));
+    if (n_obs >= SEP_MIN_OBS)
+        k_farfield_nl_sep<<<(n_obs + SEP_OBS - 1) / SEP_OBS, 32 * SEP_WARPS, 0, st>>>(
+            b, acc, fi, dl, k_wave, obs, n_obs, reinterpret_cast<double2 *>(nl));
+    else
+        k_farfield_nl<<<n_obs, FF_THREADS, 0, st>>>(b, reinterpret_cast<const double2 *>(acc), fi,
+                                                    dl, k_wave, obs, n_obs,
+                                                    reinterpret_cast<double2 *>(nl));
     count_launches(1);
     k_farfield_eh<double2><<<(n_obs + 127) / 128, 128, 0, st>>>(reinterpret_cast<const double2 *>(nl),
                                                        obs, n_obs, k_wave, eta0,

@@ -63,8 +63,7 @@ def _device_farfields(fdtd, cbox, acc, fi, freq, pts):
     capi.run("fdtd_farfield", cbox, acc.data_ptr(), int(fi), float(fdtd.dl), k_wave, float(ETA0),
              obs.data_ptr(), n_obs, nl.data_ptr(), eh.data_ptr(), q.cuda_stream)
     q.synchronize()
-    h = eh.cpu().numpy()
-    return (h[..., 0] + 1j * h[..., 1]).astype(np.complex128)
+    return eh.cpu().numpy().view(np.complex128)[..., 0]
 
 
 def _obs_array(obs_points, dtype):
@@ -339,8 +338,7 @@ class CUDANear2FarMonitor:
         capi.run("fdtd_farfield_eh", nl.data_ptr(), capi.FDTD_F32, obs.data_ptr(), n_obs, k_wave,
                  float(ETA0), eh.data_ptr(), q.cuda_stream)
         q.synchronize()
-        h = eh.cpu().numpy()
-        return (h[..., 0] + 1j * h[..., 1]).astype(np.complex128)
+        return eh.cpu().numpy().view(np.complex128)[..., 0]
 
     def get_farfield(self, obs_point, freq_index=0):
         """Far E, H at one point (metres)."""
