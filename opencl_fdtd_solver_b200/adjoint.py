@@ -154,8 +154,8 @@ class EpsilonAdjoint:
     fused_reverse    : True runs each reverse step as the TMA plane march over the
                        CPML-free interior plus CPML-shell kernels, reading one Ē/H̄
                        buffer pair and writing the other; False (default) updates Ē/H̄
-                       in place with one thread per cell, measured faster at the
-                       shell-heavy 160 x 160 x 96 configuration (143 against 152 µs per
+                       in place with grid-wide kernels, measured faster at the
+                       shell-heavy 160 x 160 x 96 configuration (76 against 152 µs per
                        reverse step).  Both give the same gradient bit for bit.
 
     The engine's own monitors are detached while this object steps it.

@@ -39,8 +39,6 @@
 
 namespace fdtd {
 
-constexpr int ADJ_TK = 32;
-constexpr int ADJ_TJ = 8;
 
 // Derivative axis of pair p (the same for the E and H orders).
 __host__ __device__ constexpr int pair_axis(int p) {
@@ -229,24 +227,238 @@ __device__ __forceinline__ void adj_e_cell(const AdjArgs<T> &a, const AdjSeed &s
     Eout[2][idx] = ez;
 }
 
-// Grid-wide reverse half steps: one thread per cell (k fastest), updating
-// in place (Hout = a.H, Hin = Eout... = a.E) or into separate outputs.
-template <typename T>
-__global__ void __launch_bounds__(ADJ_TK *ADJ_TJ)
-    k_adj_H(AdjArgs<T> a, AdjGrad<T> gb, AdjOut<T> out) {
-    const int k = blockIdx.x * ADJ_TK + threadIdx.x;
-    const int j = blockIdx.y * ADJ_TJ + threadIdx.y;
-    if (k >= a.nz || j >= a.ny) return;
-    adj_h_cell<T>(a, gb, blockIdx.z, j, k, out.H);
+// The two E pairs (H pairs) of derivative axis D at a cell: D 0: 2 and 4, 1: 0 and 5,
+// 2: 1 and 3, with fields fa, fb and coefficients ca, cb of their components.  The
+// terms and P updates of e_pair / h_pair, with the slab test, the stripe index and
+// the profile reads shared by the two and made only where the cell is in the slab.
+template <int D>
+struct AxisPairs {
+    static constexpr int A = D == 0 ? 2 : (D == 1 ? 0 : 1), B = D == 0 ? 4 : (D == 1 ? 5 : 3);
+};
+template <typename T, int D, bool OWN>
+__device__ __forceinline__ void e_axis(const AdjArgs<T> &a, int i, int j, int k, T ca, T fa, T cb,
+                                       T fb, T &ga, T &gb) {
+    constexpr int A = AxisPairs<D>::A, B = AxisPairs<D>::B;
+    constexpr bool PA = pair_pos_e(A), PB = pair_pos_e(B);
+    const int x = D == 0 ? i : (D == 1 ? j : k);
+    const T ik = a.cpe.ik[D][x];
+    const T ta = ca * ik * fa, tb = cb * ik * fb;
+    ga = PA ? ta : -ta;
+    gb = PB ? tb : -tb;
+    if (in_slab(x, D == 0 ? a.nx : (D == 1 ? a.ny : a.nz), a.npml)) {
+        const int64_t s = stripe_index<D>(i, j, k, a.nx, a.ny, a.nz, a.npml);
+        const T b = a.cpe.b[D][x], c = a.cpe.c[D][x];
+        const T ua = ca * fa, ub = cb * fb;
+        const T pa = b * a.pe[A][s] + (PA ? ua : -ua), pb = b * a.pe[B][s] + (PB ? ub : -ub);
+        if (OWN) {
+            a.pe_next[A][s] = pa;
+            a.pe_next[B][s] = pb;
+        }
+        ga = ga + c * pa;
+        gb = gb + c * pb;
+    }
+}
+template <typename T, int D, bool OWN>
+__device__ __forceinline__ void h_axis(const AdjArgs<T> &a, int i, int j, int k, T fa, T fb, T &ga,
+                                       T &gb) {
+    constexpr int A = AxisPairs<D>::A, B = AxisPairs<D>::B;
+    constexpr bool PA = !pair_pos_e(A), PB = !pair_pos_e(B);
+    const int x = D == 0 ? i : (D == 1 ? j : k);
+    const T di = a.dtm * a.cph.ik[D][x];
+    const T ta = di * fa, tb = di * fb;
+    ga = PA ? ta : -ta;
+    gb = PB ? tb : -tb;
+    if (in_slab(x, D == 0 ? a.nx : (D == 1 ? a.ny : a.nz), a.npml)) {
+        const int64_t s = stripe_index<D>(i, j, k, a.nx, a.ny, a.nz, a.npml);
+        const T b = a.cph.b[D][x], c = a.cph.c[D][x];
+        const T ua = a.dtm * fa, ub = a.dtm * fb;
+        const T pa = b * a.ph[A][s] + (PA ? ua : -ua), pb = b * a.ph[B][s] + (PB ? ub : -ub);
+        if (OWN) {
+            a.ph_next[A][s] = pa;
+            a.ph_next[B][s] = pb;
+        }
+        ga = ga + c * pa;
+        gb = gb + c * pb;
+    }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(ADJ_TK *ADJ_TJ)
-    k_adj_E(AdjArgs<T> a, AdjSeed sd, AdjOut<T> out) {
-    const int k = blockIdx.x * ADJ_TK + threadIdx.x;
-    const int j = blockIdx.y * ADJ_TJ + threadIdx.y;
-    if (k >= a.nz || j >= a.ny) return;
-    adj_e_cell<T>(a, sd, blockIdx.z, j, k, out.H, out.E);
+// Grid-wide reverse half steps, updating in place (out == a) or into separate
+// outputs.  H̄ of a cell needs the pair terms of the cell and of its +1 neighbours,
+// Ē those of its -1 neighbours.  A block owns TI x TJ x TK cells, one a thread:
+// each thread evaluates the six terms of its cell, then the halo cells beyond the
+// block's faces are shared out, two terms each, and the neighbours read them from
+// shared memory: 7.6 evaluations a cell, where a thread per cell without sharing
+// made twelve.  Bound by instructions and by the latency of L2, so by the resident
+// warps: six blocks of 256 threads an SM (40 registers).  A reverse step before /
+// after: 160x160x96 npml 12 FP32 122.7 / 75.8 us, FP64 178.9 / 113.0, 48³ npml 8
+// FP64 16.9 / 13.2, 139x88x56 npml 6 FP32 43.0 / 24.9.  Five blocks an SM 82.4 us at
+// the first of these, eight (32 registers) 73.8 but slower in FP64, 32 x 4 x 4 cells
+// 79.8; marching the block along i instead (terms of the neighbour in i carried)
+// 149.
+template <int TK, int TJ, int TI>
+struct AdjTile {
+    static constexpr int THREADS = TK * TJ * TI;
+    static constexpr int NK = TI * TJ, NJ = TI * TK, NI = TJ * TK;  // halo cells per axis
+};
+
+template <typename T, int TK, int TJ, int TI>
+__global__ void __launch_bounds__(TK *TJ *TI, 6)
+    k_adj_H(const __grid_constant__ AdjArgs<T> a, const __grid_constant__ AdjGrad<T> gb,
+            const __grid_constant__ AdjOut<T> out) {
+    using L = AdjTile<TK, TJ, TI>;
+    // terms along k (1, 3), j (0, 5) and i (2, 4), with the +1 halo
+    __shared__ T sk[2][TI][TJ][TK + 1], sj[2][TI][TJ + 1][TK], si[2][TI + 1][TJ][TK];
+    const int t = threadIdx.x;
+    const int kk = t % TK, jj = (t / TK) % TJ, ii = t / (TK * TJ);
+    const int k0 = blockIdx.x * TK, j0 = blockIdx.y * TJ, i0 = blockIdx.z * TI;
+    const int k = k0 + kk, j = j0 + jj, i = i0 + ii;
+    const int nx = a.nx, ny = a.ny, nz = a.nz;
+    const bool cell = k < nz && j < ny && i < nx;
+    const int64_t sx = (int64_t)ny * nz;
+    const int64_t idx = (int64_t)i * sx + (int64_t)j * nz + k;
+    T ex = T(0), ey = T(0), ez = T(0), hx = T(0), hy = T(0), hz = T(0);
+    T g0 = T(0), g1 = T(0), g2 = T(0), g3 = T(0), g4 = T(0), g5 = T(0);
+    if (cell) {
+        ex = a.E[0][idx];
+        ey = a.E[1][idx];
+        ez = a.E[2][idx];
+        const T cx = a.ce[0][idx], cy = a.ce[1][idx], cz = a.ce[2][idx];
+        hx = a.H[0][idx];
+        hy = a.H[1][idx];
+        hz = a.H[2][idx];
+        e_axis<T, 0, true>(a, i, j, k, cy, ey, cz, ez, g2, g4);
+        e_axis<T, 1, true>(a, i, j, k, cx, ex, cz, ez, g0, g5);
+        e_axis<T, 2, true>(a, i, j, k, cx, ex, cy, ey, g1, g3);
+    }
+    sk[0][ii][jj][kk] = g1;
+    sk[1][ii][jj][kk] = g3;
+    sj[0][ii][jj][kk] = g0;
+    sj[1][ii][jj][kk] = g5;
+    si[0][ii][jj][kk] = g2;
+    si[1][ii][jj][kk] = g4;
+    for (int t = threadIdx.x; t < L::NI + L::NJ + L::NK; t += L::THREADS) if (t < L::NI) {
+        const int hk = t % TK, hj = t / TK;
+        const int K = k0 + hk, J = j0 + hj, I = i0 + TI;
+        T p = T(0), q = T(0);
+        if (K < nz && J < ny && I < nx) {
+            const int64_t h = (int64_t)I * sx + (int64_t)J * nz + K;
+            e_axis<T, 0, false>(a, I, J, K, a.ce[1][h], a.E[1][h], a.ce[2][h], a.E[2][h], p, q);
+        }
+        si[0][TI][hj][hk] = p;
+        si[1][TI][hj][hk] = q;
+    } else if (t < L::NI + L::NJ) {
+        const int u = t - L::NI, hk = u % TK, hi = u / TK;
+        const int K = k0 + hk, J = j0 + TJ, I = i0 + hi;
+        T p = T(0), q = T(0);
+        if (K < nz && J < ny && I < nx) {
+            const int64_t h = (int64_t)I * sx + (int64_t)J * nz + K;
+            e_axis<T, 1, false>(a, I, J, K, a.ce[0][h], a.E[0][h], a.ce[2][h], a.E[2][h], p, q);
+        }
+        sj[0][hi][TJ][hk] = p;
+        sj[1][hi][TJ][hk] = q;
+    } else if (t < L::NI + L::NJ + L::NK) {
+        const int u = t - L::NI - L::NJ, hj = u % TJ, hi = u / TJ;
+        const int K = k0 + TK, J = j0 + hj, I = i0 + hi;
+        T p = T(0), q = T(0);
+        if (K < nz && J < ny && I < nx) {
+            const int64_t h = (int64_t)I * sx + (int64_t)J * nz + K;
+            e_axis<T, 2, false>(a, I, J, K, a.ce[0][h], a.E[0][h], a.ce[1][h], a.E[1][h], p, q);
+        }
+        sk[0][hi][hj][TK] = p;
+        sk[1][hi][hj][TK] = q;
+    }
+    __syncthreads();
+    if (!cell) return;
+    const T tz3 = (k >= 1 ? g3 : T(0)) - sk[1][ii][jj][kk + 1];
+    const T ty5 = (j >= 1 ? g5 : T(0)) - sj[1][ii][jj + 1][kk];
+    const T tz1 = (k >= 1 ? g1 : T(0)) - sk[0][ii][jj][kk + 1];
+    const T tx4 = (i >= 1 ? g4 : T(0)) - si[1][ii + 1][jj][kk];
+    const T ty0 = (j >= 1 ? g0 : T(0)) - sj[0][ii][jj + 1][kk];
+    const T tx2 = (i >= 1 ? g2 : T(0)) - si[0][ii + 1][jj][kk];
+    out.H[0][idx] = hx + (tz3 + ty5);
+    out.H[1][idx] = hy + (tz1 + tx4);
+    out.H[2][idx] = hz + (ty0 + tx2);
+    if (gb.active) adj_grad_cell(gb, i, j, k, ex, ey, ez);
+}
+
+template <typename T, int TK, int TJ, int TI>
+__global__ void __launch_bounds__(TK *TJ *TI, 6)
+    k_adj_E(const __grid_constant__ AdjArgs<T> a, const __grid_constant__ AdjSeed sd,
+            const __grid_constant__ AdjOut<T> out) {
+    using L = AdjTile<TK, TJ, TI>;
+    // the same with the -1 halo: index 0 is the halo
+    __shared__ T sk[2][TI][TJ][TK + 1], sj[2][TI][TJ + 1][TK], si[2][TI + 1][TJ][TK];
+    const int t = threadIdx.x;
+    const int kk = t % TK, jj = (t / TK) % TJ, ii = t / (TK * TJ);
+    const int k0 = blockIdx.x * TK, j0 = blockIdx.y * TJ, i0 = blockIdx.z * TI;
+    const int k = k0 + kk, j = j0 + jj, i = i0 + ii;
+    const int nx = a.nx, ny = a.ny, nz = a.nz;
+    const bool cell = k < nz && j < ny && i < nx;
+    const int64_t sx = (int64_t)ny * nz;
+    const int64_t idx = (int64_t)i * sx + (int64_t)j * nz + k;
+    T ex = T(0), ey = T(0), ez = T(0);
+    T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0), a4 = T(0), a5 = T(0);
+    if (cell) {
+        const T hx = out.H[0][idx], hy = out.H[1][idx], hz = out.H[2][idx];
+        ex = a.E[0][idx];
+        ey = a.E[1][idx];
+        ez = a.E[2][idx];
+        h_axis<T, 0, true>(a, i, j, k, hy, hz, a2, a4);
+        h_axis<T, 1, true>(a, i, j, k, hx, hz, a0, a5);
+        h_axis<T, 2, true>(a, i, j, k, hx, hy, a1, a3);
+    }
+    sk[0][ii][jj][kk + 1] = a1;
+    sk[1][ii][jj][kk + 1] = a3;
+    sj[0][ii][jj + 1][kk] = a0;
+    sj[1][ii][jj + 1][kk] = a5;
+    si[0][ii + 1][jj][kk] = a2;
+    si[1][ii + 1][jj][kk] = a4;
+    for (int t = threadIdx.x; t < L::NI + L::NJ + L::NK; t += L::THREADS) if (t < L::NI) {
+        const int hk = t % TK, hj = t / TK;
+        const int K = k0 + hk, J = j0 + hj, I = i0 - 1;
+        T p = T(0), q = T(0);
+        if (K < nz && J < ny && I >= 0) {
+            const int64_t h = (int64_t)I * sx + (int64_t)J * nz + K;
+            h_axis<T, 0, false>(a, I, J, K, out.H[1][h], out.H[2][h], p, q);
+        }
+        si[0][0][hj][hk] = p;
+        si[1][0][hj][hk] = q;
+    } else if (t < L::NI + L::NJ) {
+        const int u = t - L::NI, hk = u % TK, hi = u / TK;
+        const int K = k0 + hk, J = j0 - 1, I = i0 + hi;
+        T p = T(0), q = T(0);
+        if (K < nz && J >= 0 && I < nx) {
+            const int64_t h = (int64_t)I * sx + (int64_t)J * nz + K;
+            h_axis<T, 1, false>(a, I, J, K, out.H[0][h], out.H[2][h], p, q);
+        }
+        sj[0][hi][0][hk] = p;
+        sj[1][hi][0][hk] = q;
+    } else if (t < L::NI + L::NJ + L::NK) {
+        const int u = t - L::NI - L::NJ, hj = u % TJ, hi = u / TJ;
+        const int K = k0 - 1, J = j0 + hj, I = i0 + hi;
+        T p = T(0), q = T(0);
+        if (K >= 0 && J < ny && I < nx) {
+            const int64_t h = (int64_t)I * sx + (int64_t)J * nz + K;
+            h_axis<T, 2, false>(a, I, J, K, out.H[0][h], out.H[1][h], p, q);
+        }
+        sk[0][hi][hj][0] = p;
+        sk[1][hi][hj][0] = q;
+    }
+    __syncthreads();
+    if (!cell) return;
+    const T fz3 = sk[1][ii][jj][kk] - (k <= nz - 2 ? a3 : T(0));
+    const T fy5 = sj[1][ii][jj][kk] - (j <= ny - 2 ? a5 : T(0));
+    const T fz1 = sk[0][ii][jj][kk] - (k <= nz - 2 ? a1 : T(0));
+    const T fx4 = si[1][ii][jj][kk] - (i <= nx - 2 ? a4 : T(0));
+    const T fy0 = sj[0][ii][jj][kk] - (j <= ny - 2 ? a0 : T(0));
+    const T fx2 = si[0][ii][jj][kk] - (i <= nx - 2 ? a2 : T(0));
+    ex = ex + (fz3 + fy5);
+    ey = ey + (fz1 + fx4);
+    ez = ez + (fy0 + fx2);
+    if (sd.active) add_seed<T>(sd, i, j, k, ex, ey, ez);
+    out.E[0][idx] = ex;
+    out.E[1][idx] = ey;
+    out.E[2][idx] = ez;
 }
 
 // Shell reverse half steps: the cells of box o outside box b (shell_plan.cuh).
@@ -327,18 +539,26 @@ cudaError_t launch_adjoint_step(const AdjArgs<T> &a, const AdjGrad<T> &gb, const
     return launch_adjoint_grid<T>(a, gb, sd, out, st);
 }
 
-template <typename T>
-cudaError_t launch_adjoint_grid(const AdjArgs<T> &a, const AdjGrad<T> &gb, const AdjSeed &sd,
-                                const AdjOut<T> &out, cudaStream_t st) {
-    dim3 blk(ADJ_TK, ADJ_TJ, 1);
-    dim3 grd((a.nz + ADJ_TK - 1) / ADJ_TK, (a.ny + ADJ_TJ - 1) / ADJ_TJ, a.nx);
-    k_adj_H<T><<<grd, blk, 0, st>>>(a, gb, out);
+template <typename T, int TK, int TJ, int TI>
+static cudaError_t adjoint_grid_t(const AdjArgs<T> &a, const AdjGrad<T> &gb, const AdjSeed &sd,
+                                  const AdjOut<T> &out, cudaStream_t st) {
+    const dim3 grd((a.nz + TK - 1) / TK, (a.ny + TJ - 1) / TJ, (a.nx + TI - 1) / TI);
+    k_adj_H<T, TK, TJ, TI><<<grd, TK * TJ * TI, 0, st>>>(a, gb, out);
     count_launches(1);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_adj_E<T><<<grd, blk, 0, st>>>(a, sd, out);
+    k_adj_E<T, TK, TJ, TI><<<grd, TK * TJ * TI, 0, st>>>(a, sd, out);
     count_launches(1);
     return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_adjoint_grid(const AdjArgs<T> &a, const AdjGrad<T> &gb, const AdjSeed &sd,
+                                const AdjOut<T> &out, cudaStream_t st) {
+    // the narrower block where it pads nz less
+    const int w32 = (a.nz + 31) / 32 * 32, w16 = (a.nz + 15) / 16 * 16;
+    return w16 < w32 ? adjoint_grid_t<T, 16, 8, 2>(a, gb, sd, out, st)
+                     : adjoint_grid_t<T, 32, 4, 2>(a, gb, sd, out, st);
 }
 
 template <typename T>
