@@ -111,28 +111,31 @@ def edge_to_cells(G, eps_full, design, box):
     ``ce = dt/(ε0·ε_edge)`` gives ``∂J/∂ε_edge = −G/ε_edge``; ``ε_edge`` is the mean of
     the two cells sharing the edge, the last plane keeping the cell value
     (reference ``materials.py:28-41``), so each cell collects half of its two edges
-    along each axis (all of the last-plane edge).
+    along each axis (all of the last-plane edge).  Only the box and the plane after
+    it are touched.
     """
-    eps_e = _edge_eps(eps_full)
-    shape = eps_full.shape
-    bsl = tuple(slice(lo, hi) for lo, hi in box)
-    dsl = tuple(slice(lo, hi) for lo, hi in design)
+    eps_e = _edge_eps(eps_full[tuple(slice(lo, hi + 1) for lo, hi in box)])
+    ext = tuple(slice(0, hi - lo) for lo, hi in box)
+    inner = tuple(slice(lo - b, hi - b) for (lo, hi), (b, _) in zip(design, box))
     out = np.zeros(tuple(hi - lo for lo, hi in design), np.float64)
     for c in range(3):
-        ge = np.zeros(shape, np.float64)
-        ge[bsl] = -G[c] / eps_e[c][bsl]
-        n = shape[c]
-        cell = np.zeros(shape, np.float64)
-        dst = [slice(None)] * 3
-        src = [slice(None)] * 3
-        dst[c] = slice(0, n - 1)
-        cell[tuple(dst)] += 0.5 * ge[tuple(dst)]      # edge i   -> cell i
-        dst[c] = slice(1, n)
-        src[c] = slice(0, n - 1)
-        cell[tuple(dst)] += 0.5 * ge[tuple(src)]      # edge i-1 -> cell i
-        dst[c] = slice(n - 1, n)
-        cell[tuple(dst)] += ge[tuple(dst)]            # last plane
-        out += cell[dsl]
+        ge = -G[c] / eps_e[c][ext]
+        n = eps_full.shape[c]
+        (d0, d1), b0 = design[c], box[c][0]
+
+        def on_axis(rest, lo, hi):
+            return tuple(slice(lo, hi) if a == c else rest[a] for a in range(3))
+
+        cell = np.zeros_like(out)
+        full = (slice(None),) * 3
+        own = min(d1, n - 1)       # edge i of the cells i < n - 1
+        cell[on_axis(full, 0, own - d0)] += 0.5 * ge[on_axis(inner, d0 - b0, own - b0)]
+        low = max(d0, 1)           # edge i - 1 of the cells i >= 1
+        cell[on_axis(full, low - d0, d1 - d0)] += \
+            0.5 * ge[on_axis(inner, low - 1 - b0, d1 - 1 - b0)]
+        if d1 == n:                # the last plane's own edge
+            cell[on_axis(full, n - 1 - d0, n - d0)] += ge[on_axis(inner, n - 1 - b0, n - b0)]
+        out += cell
     return out
 
 
