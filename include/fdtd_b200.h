@@ -254,8 +254,9 @@ int fdtd_n2f_workspace(const fdtd_n2f_face *faces, int32_t nfaces, int32_t nfreq
  * dirs: device, n_obs unit vectors (float64 xyz); nl: device, complex64
  * [nfreq][n_obs][6] for the tensor-core modes, complex128 for FDTD_N2F_FP64.
  * The tensor-core modes pack the currents into the workspace (256-byte
- * aligned), run one CTA per (128 directions, face, frequency) and reduce the
- * faces; bounded waits set bit 1 of fdtd_device_status on timeout. */
+ * aligned; split-BF16 packs the sums and differences of the samples about each
+ * face's middle), run one CTA per (128 directions, one or more faces, frequency)
+ * and reduce the faces; bounded waits set bit 1 of fdtd_device_status on timeout. */
 int fdtd_n2f_contract(const fdtd_n2f_face *faces, int32_t nfaces, int32_t cur_dtype,
                       const double *freqs, int32_t nfreq, const double *dirs, int32_t n_obs,
                       int32_t mode, void *workspace, uint64_t workspace_bytes, void *nl,

@@ -382,7 +382,6 @@ int plan_n2f(const fdtd_n2f_face *faces, int nfaces, int nfreq, int n_obs, int m
     P.n_obs = n_obs;
     P.nfaces = nfaces;
     const bool tc = mode != FDTD_N2F_FP64;
-    const int kr = tc ? fdtd::n2f::k_real_per_step(mode) : 16;
     const int64_t bcopy = tc ? fdtd::n2f::b_copy_bytes(mode) : 0;
     uint64_t off = 0;
     for (int f = 0; f < nfaces; ++f) {
@@ -399,8 +398,7 @@ int plan_n2f(const fdtd_n2f_face *faces, int nfaces, int nfreq, int n_obs, int m
         G.axis_q = F.normal == 2 ? 1 : 2;
         G.np = F.np;
         G.nq = F.nq;
-        G.ks = (2 * F.np + kr - 1) / kr;
-        G.nt = (F.nq + fdtd::n2f::QT - 1) / fdtd::n2f::QT;
+        if (tc) fdtd::n2f::operand_steps(mode, F.np, F.nq, G.ks, G.nt);
         G.x_n = F.x_n;
         G.o_p = F.o_p;
         G.o_q = F.o_q;
@@ -805,15 +803,9 @@ int fdtd_n2f_contract(const fdtd_n2f_face *faces, int32_t nfaces, int32_t cur_dt
     if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
         return fail(FDTD_ERR_INVALID, "workspace must be 256-byte aligned");
     unsigned char *ws = (unsigned char *)workspace;
-    for (int f = 0; f < nfaces; ++f) {
-        const auto &G = P.face[f];
-        e = cur_dtype == FDTD_F32
-                ? fdtd::n2f::launch_pack<float2>(mode, (const float2 *)P.cur[f], nfreq, G.np, G.nq,
-                                                 G.ks, G.nt, ws + G.b_off, st)
-                : fdtd::n2f::launch_pack<double2>(mode, (const double2 *)P.cur[f], nfreq, G.np,
-                                                  G.nq, G.ks, G.nt, ws + G.b_off, st);
-        if (e != cudaSuccess) return cuda_status(e, "n2f_pack");
-    }
+    e = cur_dtype == FDTD_F32 ? fdtd::n2f::launch_pack<float2>(mode, P, nfreq, ws, st)
+                              : fdtd::n2f::launch_pack<double2>(mode, P, nfreq, ws, st);
+    if (e != cudaSuccess) return cuda_status(e, "n2f_pack");
     P.btiles = ws;
     P.partial = (float2 *)(ws + pl.partial_off);
     if ((e = fdtd::n2f::launch_contract(mode, P, nfreq, st)) != cudaSuccess)

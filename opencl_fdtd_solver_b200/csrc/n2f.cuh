@@ -10,7 +10,8 @@ namespace fdtd {
 namespace n2f {
 
 constexpr int BM = 128;  // directions per CTA (TMEM lanes)
-constexpr int BN = 256;  // real accumulator columns per n tile: 32 q x 4 currents x (Re, Im)
+constexpr int BN = 256;  // real accumulator columns per n tile: 32 q, or 16 q pairs x (even,
+                         // odd), x 4 currents x (Re, Im)
 constexpr int QT = 32;   // samples q per n tile
 
 struct Face {
@@ -23,6 +24,7 @@ struct Face {
 
 struct Params {
     int n_obs, nfaces;
+    int face_group;       // faces per CTA of the contraction kernel
     const double *dirs;   // [n_obs][3] unit vectors (device)
     const double *freqs;  // [nfreq] (device)
     Face face[6];
@@ -35,10 +37,11 @@ struct Params {
 
 size_t stage_smem(int mode, bool atm);
 int b_copy_bytes(int mode);
-int k_real_per_step(int mode);
+// K steps and n tiles of the packed operand of an np x nq face.
+void operand_steps(int mode, int np, int nq, int &ks, int &nt);
 template <typename CT>
-cudaError_t launch_pack(int mode, const CT *cur, int nfreq, int np, int nq, int KS, int NT,
-                        unsigned char *dst, cudaStream_t st);
+cudaError_t launch_pack(int mode, const Params &P, int nfreq, unsigned char *dst,
+                        cudaStream_t st);
 cudaError_t launch_contract(int mode, const Params &P, int nfreq, cudaStream_t st);
 cudaError_t launch_combine(const Params &P, int nfreq, float2 *nl, cudaStream_t st);
 template <typename CT>
