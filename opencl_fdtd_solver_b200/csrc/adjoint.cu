@@ -32,6 +32,7 @@
 
 #include <cstdint>
 
+#include "launch_chain.cuh"
 #include "launch_count.cuh"
 #include "../../include/fdtd_b200.h"
 #include "adjoint.cuh"
@@ -305,6 +306,8 @@ template <typename T, int TK, int TJ, int TI>
 __global__ void __launch_bounds__(TK *TJ *TI, 6)
     k_adj_H(const __grid_constant__ AdjArgs<T> a, const __grid_constant__ AdjGrad<T> gb,
             const __grid_constant__ AdjOut<T> out) {
+    chain_next();
+    chain_wait();
     using L = AdjTile<TK, TJ, TI>;
     // terms along k (1, 3), j (0, 5) and i (2, 4), with the +1 halo
     __shared__ T sk[2][TI][TJ][TK + 1], sj[2][TI][TJ + 1][TK], si[2][TI + 1][TJ][TK];
@@ -385,6 +388,8 @@ template <typename T, int TK, int TJ, int TI>
 __global__ void __launch_bounds__(TK *TJ *TI, 6)
     k_adj_E(const __grid_constant__ AdjArgs<T> a, const __grid_constant__ AdjSeed sd,
             const __grid_constant__ AdjOut<T> out) {
+    chain_next();
+    chain_wait();
     using L = AdjTile<TK, TJ, TI>;
     // the same with the -1 halo: index 0 is the halo
     __shared__ T sk[2][TI][TJ][TK + 1], sj[2][TI][TJ + 1][TK], si[2][TI + 1][TJ][TK];
@@ -518,6 +523,8 @@ __global__ void k_adj_seed(int nx, int ny, int nz, T *E0, T *E1, T *E2, AdjSeed 
 template <typename T>
 __global__ void k_capture(int ny, int nz, const T *E0, const T *E1, const T *E2, int3 lo,
                           int3 ext, T *out) {
+    chain_next();
+    chain_wait();
     const int plane_cells = ext.y * ext.z;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= plane_cells) return;
@@ -543,13 +550,13 @@ template <typename T, int TK, int TJ, int TI>
 static cudaError_t adjoint_grid_t(const AdjArgs<T> &a, const AdjGrad<T> &gb, const AdjSeed &sd,
                                   const AdjOut<T> &out, cudaStream_t st) {
     const dim3 grd((a.nz + TK - 1) / TK, (a.ny + TJ - 1) / TJ, (a.nx + TI - 1) / TI);
-    k_adj_H<T, TK, TJ, TI><<<grd, TK * TJ * TI, 0, st>>>(a, gb, out);
+    cudaError_t e =
+        launch_chained(k_adj_H<T, TK, TJ, TI>, grd, TK * TJ * TI, 0, st, a, gb, out);
     count_launches(1);
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_adj_E<T, TK, TJ, TI><<<grd, TK * TJ * TI, 0, st>>>(a, sd, out);
+    e = launch_chained(k_adj_E<T, TK, TJ, TI>, grd, TK * TJ * TI, 0, st, a, sd, out);
     count_launches(1);
-    return cudaGetLastError();
+    return e;
 }
 
 template <typename T>
@@ -613,9 +620,10 @@ cudaError_t launch_capture(int ny, int nz, const T *const E[3], const int lo[3],
         return cudaErrorInvalidValue;
     const int thr = 256;
     const dim3 grid((unsigned)(((int64_t)ext.y * ext.z + thr - 1) / thr), (unsigned)(3 * ext.x), 1);
-    k_capture<T><<<grid, thr, 0, st>>>(ny, nz, E[0], E[1], E[2], l, ext, out);
+    const cudaError_t e =
+        launch_chained(k_capture<T>, grid, thr, 0, st, ny, nz, E[0], E[1], E[2], l, ext, out);
     count_launches(1);
-    return cudaGetLastError();
+    return e;
 }
 
 template cudaError_t launch_adjoint_step<float>(const AdjArgs<float> &, const AdjGrad<float> &,

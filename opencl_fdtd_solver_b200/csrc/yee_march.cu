@@ -39,6 +39,7 @@
 #include <cstdint>
 #include <cstring>
 
+#include "launch_chain.cuh"
 #include "launch_count.cuh"
 #include "tma.cuh"
 #include "yee_launch.cuh"
@@ -652,6 +653,8 @@ template <typename T, typename L, bool LOSSY>
 __global__ void __launch_bounds__(L::THREADS, 2)
     k_march(const __grid_constant__ MarchMaps maps, const __grid_constant__ YeeArgs<T> a,
             const __grid_constant__ MarchBox bx, const __grid_constant__ SourceList src) {
+    chain_next();
+    chain_wait();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
@@ -820,9 +823,9 @@ cudaError_t launch_march_t(const YeeArgs<T> &a, const SourceList &src, cudaStrea
     cudaError_t e = ensure_max_dynamic_smem((const void *)k_march<T, L, LOSSY>, L::SMEM);
     if (e != cudaSuccess) return e;
     const unsigned ctas = (unsigned)(bx.tiles * (bx.nmid + bx.nlo + bx.nhi));
-    k_march<T, L, LOSSY><<<ctas, L::THREADS, L::SMEM, st>>>(maps, a, bx, src);
+    e = launch_chained(k_march<T, L, LOSSY>, ctas, L::THREADS, L::SMEM, st, maps, a, bx, src);
     count_launches(1);
-    return cudaGetLastError();
+    return e;
 }
 
 // 64 x 8 (FP64: 32 x 8) streams better; the narrower tile is taken where it saves

@@ -26,6 +26,7 @@
 // decoded with multiply-high divisions (consecutive threads take consecutive k).
 #include <cuda_runtime.h>
 
+#include "launch_chain.cuh"
 #include "launch_count.cuh"
 #include "shell_plan.cuh"
 #include "yee_launch.cuh"
@@ -36,6 +37,8 @@ namespace fdtd {
 template <typename T>
 __global__ void __launch_bounds__(SHELL_THREADS)
     k_shell_H(YeeArgs<T> a, ShellPlan sp) {
+    chain_next();
+    chain_wait();
     const int nx = a.nx, ny = a.ny, nz = a.nz, npml = a.npml;
     int i, j, k;
     if (!shell_cell(blockIdx.x * SHELL_THREADS + threadIdx.x, sp, i, j, k)) return;
@@ -102,6 +105,8 @@ __device__ __forceinline__ void shell_E_cell(const YeeArgs<T> &a, int i, int j, 
 template <typename T, bool LOSSY>
 __global__ void __launch_bounds__(SHELL_THREADS)
     k_shell_E(YeeArgs<T> a, ShellPlan sp, SourceList src, const __grid_constant__ PlaneList planes) {
+    chain_next();
+    chain_wait();
     int i, j, k;
     if (!shell_cell(blockIdx.x * SHELL_THREADS + threadIdx.x, sp, i, j, k)) return;
     shell_E_cell<T, LOSSY>(a, i, j, k, src, planes);
@@ -124,6 +129,8 @@ __global__ void __launch_bounds__(SHELL_THREADS)
 template <typename T>
 __global__ void __launch_bounds__(SHELL_THREADS)
     k_plane_dft_box(YeeArgs<T> a, ShellBox b, PlaneList planes, int q) {
+    chain_next();
+    chain_wait();
     const fdtd_plane_dft &p = planes.p[q];
     const int ax = p.axis, u = (ax == 0) ? 1 : 0, w = (ax == 2) ? 1 : 2;
     const int nu = b.hi[u] - b.lo[u], nw = b.hi[w] - b.lo[w];
@@ -154,11 +161,13 @@ cudaError_t launch_plane_dft_box(const YeeArgs<T> &a, const ShellBox &b, const P
         if (pl.p[q].index < b.lo[ax] || pl.p[q].index >= b.hi[ax]) continue;
         const int64_t n = (int64_t)(b.hi[u] - b.lo[u]) * (b.hi[w] - b.lo[w]);
         if (n <= 0) continue;
-        k_plane_dft_box<T><<<(unsigned)((n + SHELL_THREADS - 1) / SHELL_THREADS), SHELL_THREADS, 0,
-                             st>>>(a, b, pl, q);
+        const cudaError_t e =
+            launch_chained(k_plane_dft_box<T>, (unsigned)((n + SHELL_THREADS - 1) / SHELL_THREADS),
+                           SHELL_THREADS, 0, st, a, b, pl, q);
+        if (e != cudaSuccess) return e;
         count_launches(1);
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 template cudaError_t launch_plane_dft_box<float>(const YeeArgs<float> &, const ShellBox &,
@@ -173,9 +182,9 @@ cudaError_t launch_shell_H(const YeeArgs<T> &a, const ShellBox &b, cudaStream_t 
     const ShellPlan sp = make_plan(o, b);
     const unsigned nb = shell_blocks(sp);
     if (nb == 0) return cudaSuccess;
-    k_shell_H<T><<<nb, SHELL_THREADS, 0, st>>>(a, sp);
+    const cudaError_t e = launch_chained(k_shell_H<T>, nb, SHELL_THREADS, 0, st, a, sp);
     count_launches(1);
-    return cudaGetLastError();
+    return e;
 }
 
 template <typename T>
@@ -185,12 +194,10 @@ cudaError_t launch_shell_E_region(const YeeArgs<T> &a, const ShellBox &o, const 
     const ShellPlan sp = make_plan(o, b);
     const unsigned nb = shell_blocks(sp);
     if (nb == 0) return cudaSuccess;
-    if (a.lossy)
-        k_shell_E<T, true><<<nb, SHELL_THREADS, 0, st>>>(a, sp, src, pl);
-    else
-        k_shell_E<T, false><<<nb, SHELL_THREADS, 0, st>>>(a, sp, src, pl);
+    const cudaError_t e = launch_chained(a.lossy ? k_shell_E<T, true> : k_shell_E<T, false>, nb,
+                                         SHELL_THREADS, 0, st, a, sp, src, pl);
     count_launches(1);
-    return cudaGetLastError();
+    return e;
 }
 
 template <typename T>
