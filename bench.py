@@ -1049,10 +1049,10 @@ def run_kernels_leg(args):
     """One launch (after warm-up) of each auxiliary kernel at documented sizes,
     timed by CUDA events; the workload of the per-kernel ncu summaries.
       * medium configuration (256³, npml 12): one fused step with the Huygens box
-        (k_shell_H, k_interior, k_plane_dft_box, k_shell_E, k_dft_faces) and one
+        (k_march, k_plane_dft_box, k_dft_faces) and one
         split step (k_update_H, k_update_E), with a z-plane DFT of Ex at 4 freqs;
       * the far field of the box at one frequency onto 181 x 91 directions
-        (k_farfield_nl, k_farfield_eh);
+        (k_farfield_nl_sep, k_farfield_eh);
       * the tensor-core contraction of a 160³ box (6 faces, 4 currents, 8 freqs)
         onto 361 x 181 directions in split-BF16 (k_n2f_pack, k_n2f_tc, k_n2f_combine)."""
     import torch

@@ -807,15 +807,18 @@ static cudaError_t launch_step_grid(const YeeArgs<T> &a, const SourceList &src,
     return e;
 }
 
-// Grids of this many cells that no march takes run as the two whole-grid
-// launches where these beat the interior march with shell kernels: small grids,
-// lossy ones with much CPML, and those whose z slabs (short rows for the shell
-// kernels) hold two fifths of the grid.  Measured per step, two launches / interior march, in us: FP32 with
-// a source and a plane DFT 48³ 13.5 / 24.7, 64³ 16.4 / 25.3, 96³ 28.0 / 31.4, 128³
-// 59.7 / 60.5; without, 46x445x288 npml 10 lossy 142.3 / 145.8, 300x300x60 npml 20
-// 133.0 / 163.8, 34x483x224 npml 13 96.1 / 96.3, 64x376x144 npml 16 88.3 / 84.9.
+// Grids of this many cells that the march does not take run as the two whole-grid
+// launches: those whose step fits the L2, lossy ones, those whose z slabs (short rows
+// for the shell kernels) hold two fifths of the rows, and, unless interior_pays or
+// interior_beats_grid, all that could have marched (a second ψ_H given).  The interior
+// march with shell kernels keeps the rest.  Measured per step, two launches / interior
+// march, in us: FP32 with a
+// source and a plane DFT 48³ 13.5 / 24.7, 64³ 16.4 / 25.3, 96³ 28.0 / 31.4; lossy FP32
+// 280x216x80 npml 6 110 / 158, 256³ npml 12 336 / 381, FP64 160³ npml 4 142 / 176, 384³
+// npml 16 1840 / 1993; lossless FP32 300x300x60 npml 20 133.0 / 163.8, 160x160x96 npml 12
+// 58.5 / 65.6, but 384³ FP64 npml 16 1733 / 1535 for a caller that steps in place.
 // The two launches win below the line too (40x36x48 14.3 / 27.3), but the bounded
-// waits of the interior march and its launch counts are checked on such a grid.
+// waits of the interior march and its launch counts are tested on such a grid.
 constexpr int64_t GRID_MIN_CELLS = 100000;
 
 template <typename T>
@@ -828,11 +831,13 @@ cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const 
         if (e != cudaErrorNotSupported) return e;  // else no tensor maps, nothing launched
     }
     const int64_t cells = (int64_t)a.nx * a.ny * a.nz;
+    const bool swap = a.psi_h_next[0] != a.psi_h[0];
     if (face_mode() != 1 && cells >= GRID_MIN_CELLS &&
         (!march_size<T>(cells) ||
          (!a.ghost_lo && !a.ghost_hi &&
-          (5 * a.npml >= a.nz ||
-           (a.lossy && pml_fraction(a.nx, a.ny, a.nz, a.npml) >= 0.4)))))
+          (5 * a.npml >= a.nz || a.lossy ||
+           (swap && !interior_pays(a.nx, a.nz, a.npml, march_pad<T>(a.ny, a.nz)) &&
+            !interior_beats_grid<T>(a.nx, a.ny, a.nz, a.npml))))))
         return launch_step_grid<T>(a, src, pl, st);
     // interior H box B = [npml, N-npml)^3 (x on a slab: [pml_lo, nx - pml_hi -
     // ghost_hi), so the upper ghost plane, whose forward differences would read

@@ -84,17 +84,65 @@ inline bool march_size(int64_t cells) {
     return 15 * cells * (int64_t)sizeof(T) >= MARCH_MIN_BYTES;
 }
 
-// And whose CPML is not most of the grid: its CPML tiles evaluate their cells in
-// fewer, longer threads.  In ps per FP32 cell the march costs about (11 + 20 f)
-// per cell of its (padded) tiles, f the CPML fraction, 1.17 times that with ca; the
-// two whole-grid launches 21 + 4 f, 1.08 times with ca.  Measured, march / whole-grid
-// launches in us: 256³ npml 20 lossy (f 0.40) 349.9 / 363.9, 192³ npml 20 lossy
-// (0.50) 161 / 171, 100x300x200 npml 20 (0.58) 154.4 / 137.5, 160³ npml 20 lossy
-// (0.58) 124.2 / 108.6, 34x483x224 npml 13 (0.80) 117.8 / 94.6.
-inline bool march_pays(int nx, int ny, int nz, int npml, bool lossy, int tk, int tj) {
-    const double pad = (double)((nz + tk - 1) / tk * tk) / nz * ((ny + tj - 1) / tj * tj) / ny;
-    const double f = pml_fraction(nx, ny, nz, npml);
-    return pad * (11.0 + 20.0 * f) * (lossy ? 1.17 : 1.0) < (21.0 + 4.0 * f) * (lossy ? 1.08 : 1.0);
+// Padding of a grid's (j, k) plane to whole tiles.
+inline double tile_pad(int ny, int nz, int tk, int tj) {
+    return (double)((nz + tk - 1) / tk * tk) / nz * ((ny + tj - 1) / tj * tj) / ny;
+}
+
+// Lossless grids that the march's tiles pad and whose z slabs are a tenth of the rows
+// at most stay with the interior march and its shell kernels, if the planes are few.
+// Per step in us, interior march / march / two whole-grid launches: FP32 72x224x328
+// npml 4 82.1 / 96.0 / 94.5, 200³ npml 4 126.8 / 142.7 / 139.7, 328x224x208 npml 8 234 /
+// 245 / 266, but 368x224x272 npml 4 345 / 316 / 370; FP64 48x292x104 npml 4 54.3 / 62.6 /
+// 54.9, 120x239x136 npml 4 115 / 127 / 129, but 355x136x52 npml 6 117.8 / 91.6 / 95.2.
+inline bool interior_pays(int nx, int nz, int npml, double pad) {
+    return pad > 1.05 && nz >= 20 * npml && (nx <= 256 || pad > 1.2);
+}
+
+// And those, not for the march, with long rows, enough cells and little CPML: FP32,
+// interior march / two whole-grid launches, 84x296x264 npml 10 120 / 129, 62x200x352 npml
+// 8 82.6 / 86.8, 328x224x208 npml 8 234 / 266; but 150x136x176 npml 10 78.6 / 74.7,
+// 280x216x80 npml 6 127 / 99, 192³ npml 20 157 / 149.
+template <typename T>
+inline bool interior_beats_grid(int nx, int ny, int nz, int npml) {
+    const int64_t cells = (int64_t)nx * ny * nz;
+    return nz * (int)sizeof(T) >= 768 && cells * (int)sizeof(T) >= 16000000 &&
+           pml_fraction(nx, ny, nz, npml) <= 0.42;
+}
+
+// Where the march beats the two whole-grid launches.  Its CPML tiles evaluate their
+// cells in fewer, longer threads, its padding is work, and the narrower tile streams
+// less well in FP32.  In ps per cell, f the CPML fraction, lossless FP32 grids below
+// 10 M cells take about pad (11 + 20 f), 1.45 times that in narrow tiles, against 18 +
+// 7 f; measured, march / whole-grid launches in us: 192³ npml 20 132 / 149, 160x160x96
+// npml 12 (narrow) 63.7 / 58.5, 280x216x80 npml 6 (narrow) 145.8 / 99.0, 240x48x280 npml
+// 10 97 / 72, 150x136x176 npml 10 82.2 / 74.7.  Above, the bytes count: 344x136x272 npml
+// 16 216 / 241, 398x160x336 npml 20 351 / 404.  FP64: 192³ npml 8 194.5 / 227.6,
+// 34x483x224 npml 13 172 / 158, 384³ npml 16 1365 / 1733.  Lossy (a deeper read per cell,
+// one stage less in the ring): 192³ npml 20 158 / 164, 256³ npml 12 327 / 336, but padded
+// 200³ npml 4 194.9 / 157.6 and FP64 192³ npml 8 268.5 / 240.6.
+template <typename T>
+inline bool march_pays(int nx, int ny, int nz, int npml, bool lossy, bool narrow, double pad) {
+    const int64_t cells = (int64_t)nx * ny * nz;
+    if (lossy) return sizeof(T) == 4 && !narrow && pad < 1.05 && cells >= 7000000;
+    if (interior_pays(nx, nz, npml, pad)) return false;
+    const double f = pml_fraction(nx, ny, nz, npml), march = pad * (11.0 + 20.0 * f);
+    if (sizeof(T) == 8) return march < 21.0 + 4.0 * f;
+    if (!narrow && cells >= 10000000) return f < 0.6;
+    return (narrow ? 1.45 : 1.0) * march < 18.0 + 7.0 * f;
+}
+
+// Tile of a grid's march: 64 x 8 (FP64: 32 x 8) cells streams better; the narrower one
+// is taken where it saves a fifth of the padded k extent.
+template <typename T>
+inline bool march_narrow(int nz) {
+    constexpr int W = 256 / (int)sizeof(T), N = W / 2;
+    return 5 * ((nz + W - 1) / W * W) > 6 * ((nz + N - 1) / N * N);
+}
+template <typename T>
+inline double march_pad(int ny, int nz) {
+    const bool narrow = march_narrow<T>(nz);
+    return tile_pad(ny, nz, (narrow ? 128 : 256) / (int)sizeof(T), narrow ? 16 : 8);
 }
 
 // The whole step but the plane DFTs as one plane march over the grid, CPML

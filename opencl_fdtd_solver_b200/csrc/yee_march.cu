@@ -828,14 +828,6 @@ cudaError_t launch_march_t(const YeeArgs<T> &a, const SourceList &src, cudaStrea
     return e;
 }
 
-// 64 x 8 (FP64: 32 x 8) streams better; the narrower tile is taken where it saves
-// a fifth of the padded k extent.
-template <typename T>
-bool march_narrow(int nz) {
-    constexpr int W = 256 / (int)sizeof(T), N = W / 2;
-    return 5 * ((nz + W - 1) / W * W) > 6 * ((nz + N - 1) / N * N);
-}
-
 bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 }  // namespace
@@ -859,20 +851,19 @@ bool march_path_ok(const YeeArgs<T> &a) {
             !aligned16(a.H_next[c]) || !aligned16(a.ce[c]) || (a.lossy && !aligned16(a.ca[c])))
             return false;
     if (!march_size<T>((int64_t)a.nx * a.ny * a.nz)) return false;
-    const bool narrow = march_narrow<T>(a.nz);
-    const int tk = (narrow ? 128 : 256) / (int)sizeof(T), tj = narrow ? 16 : 8;
-    return march_pays(a.nx, a.ny, a.nz, P, a.lossy != 0, tk, tj);
+    return march_pays<T>(a.nx, a.ny, a.nz, P, a.lossy != 0, march_narrow<T>(a.nz),
+                         march_pad<T>(a.ny, a.nz));
 }
 
 // cudaErrorNotSupported, with nothing launched, when the tensor maps cannot be built.
 template <typename T>
 cudaError_t launch_march(const YeeArgs<T> &a, const SourceList &src, cudaStream_t st) {
     constexpr int W = 256 / (int)sizeof(T), N = W / 2;
-    if (march_narrow<T>(a.nz))
-        return a.lossy ? launch_march_t<T, N, 16, true>(a, src, st)
-                       : launch_march_t<T, N, 16, false>(a, src, st);
-    return a.lossy ? launch_march_t<T, W, 8, true>(a, src, st)
-                   : launch_march_t<T, W, 8, false>(a, src, st);
+    // march_pays: lossy grids in FP32 and the wide tile only
+    if (march_narrow<T>(a.nz)) return launch_march_t<T, N, 16, false>(a, src, st);
+    if constexpr (sizeof(T) == 4)
+        if (a.lossy) return launch_march_t<T, W, 8, true>(a, src, st);
+    return launch_march_t<T, W, 8, false>(a, src, st);
 }
 
 template bool march_path_ok<float>(const YeeArgs<float> &);

@@ -25,15 +25,18 @@ FIELDS = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
 CASES = [
     # shape, npml, lossy
     ((220, 170, 64), 4, False),      # one tile along k
-    ((137, 175, 104), 5, True),      # partial tiles; vectors straddle the z slabs' edges
+    ((137, 175, 104), 5, True),      # lossy, odd npml: two whole-grid launches
     ((150, 186, 92), 6, False),      # straddling in FP32 only
-    ((230, 131, 96), 3, True),       # narrow tile, many planes: several chunks
+    ((230, 131, 96), 3, True),       # lossy: two whole-grid launches
     ((26, 680, 140), 2, False),      # few planes; slab ends inside a tile
     ((244, 250, 64), 12, False),     # a rim row in the next tile
     ((1000, 47, 60), 1, False),      # one CPML layer
+    ((192, 192, 192), 5, True),      # lossy march (FP32); vectors straddle the z slabs' edges
+    ((320, 160, 96), 2, False),      # narrow tile in FP32, many planes: several chunks
+    ((72, 224, 160), 4, False),      # padded, few planes: interior march and shell kernels
     ((181, 142, 103), 9, True),      # odd rows: two whole-grid launches
     ((46, 445, 120), 16, True),      # mostly CPML, lossy: two whole-grid launches
-    ((90, 320, 84), 12, False),      # mostly CPML, lossless: interior march and shell kernels
+    ((90, 320, 84), 12, False),      # mostly CPML, lossless: two whole-grid launches
     ((70, 60, 56), 6, False),        # small: two whole-grid launches
 ]
 
