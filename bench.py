@@ -341,9 +341,16 @@ def run_steps_timed(g, k):
     ms = (ctypes.c_double * 5)()
     nsteps = ctypes.c_int32()
     capi.run("fdtd_profile_read", ms, ctypes.byref(nsteps))
-    per_kernel = {name: ms[i] / max(1, nsteps.value)
-                  for i, name in enumerate(("k_shell_H", "k_shell_E_side", "k_interior",
-                                            "k_plane_dft_box", "k_shell_E"))}
+    by_sched = (ctypes.c_int32 * capi.FDTD_SCHEDULES)()
+    capi.run("fdtd_profile_schedules", by_sched)
+    # the profile's slots, by the schedule that the steps took (none: split kernels)
+    slots = {capi.FDTD_SCHEDULE_MARCH: {2: "k_march", 3: "k_plane_dft_box"},
+             capi.FDTD_SCHEDULE_GRID: {0: "k_shell_H", 4: "k_shell_E"}}
+    interior = dict(enumerate(("k_shell_H", "k_shell_E_side", "k_interior", "k_plane_dft_box",
+                               "k_shell_E")))
+    sched = max(range(capi.FDTD_SCHEDULES), key=lambda s: by_sched[s])
+    per_kernel = {name: ms[i] / nsteps.value
+                  for i, name in slots.get(sched, interior).items()} if nsteps.value else {}
     phases = {f"ms_per_step_first_{split}": round(start.elapsed_time(mid) / max(1, split), 4)}
     if k > split:
         phases[f"ms_per_step_after_{split}"] = round(mid.elapsed_time(end) / (k - split), 4)
@@ -377,20 +384,20 @@ def run_b200_arm(args, rank, world, local):
     peak, peak_kind = measured_hbm()
     bpc = alg_bytes_per_cell(shape, npml, item, ((2, 1, len(FREQS)),))
     step_achieved = bpc * cells / (ms_per_step / 1e3) / 1e9
-    if fused and launches <= 2 * args.steps:
-        # one march over the whole grid (timed in the interior kernel's slot), then
-        # the plane DFT
-        k_ms = per_kernel.pop("k_interior")
-        per_kernel = {"k_march": k_ms, "k_plane_dft_box": per_kernel["k_plane_dft_box"]}
+    if "k_march" in per_kernel:
+        # one march over the whole grid, then the plane DFT
+        k_ms = per_kernel["k_march"]
         k_bytes = alg_bytes_per_cell(shape, npml, item, ()) * cells
         kname = "k_march"
-    elif fused and per_kernel["k_interior"] > 0:
+    elif "k_interior" in per_kernel:
         # dominant kernel: the interior single-pass kernel (largest share of the step)
         k_ms = per_kernel["k_interior"]
         k_bytes = interior_alg_bytes(shape, npml, item)
         kname = "k_interior"
     else:
-        kname, k_ms, k_bytes = "step (split kernels)", ms_per_step, bpc * cells
+        # two launches over the whole grid, the plane DFT in the second
+        kname = "k_shell_H + k_shell_E" if per_kernel else "step (split kernels)"
+        k_ms, k_bytes = sum(per_kernel.values()) or ms_per_step, bpc * cells
     achieved = k_bytes / (k_ms / 1e3) / 1e9
     traffic = None
     tp = ROOT / "profiles" / "yee_step_traffic.json"

@@ -154,6 +154,19 @@ int fdtd_step_swap(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
                    const fdtd_source *src, int32_t nsrc,
                    const fdtd_plane_dft *planes, int32_t nplanes, void *stream);
 
+/* How a fused step runs: one march over every cell, then the plane DFTs; two
+ * launches over every cell (H, then E with the DFTs fused); the interior march
+ * beside per-cell kernels for the CPML shell; the same with the shell's E by the
+ * CPML face marches.  fdtd_step_schedule tells which one fdtd_step (swap == 0) or
+ * fdtd_step_swap (swap != 0) takes for a grid whose buffers lie on 16-byte
+ * boundaries.  It runs on the host alone.  No reference counterpart. */
+#define FDTD_SCHEDULE_MARCH 0
+#define FDTD_SCHEDULE_GRID 1
+#define FDTD_SCHEDULE_INTERIOR 2
+#define FDTD_SCHEDULE_FACES 3
+#define FDTD_SCHEDULES 4
+int fdtd_step_schedule(const fdtd_grid *g, int32_t swap, int32_t *schedule);
+
 /* Immediate sheet injection into Ex (used when a source callback reads fields
  * after injecting).  Replaces add_source_Jx / add_source_Ex
  * (sources.cl:7-49, engine.py:448-538). */
@@ -373,20 +386,24 @@ int fdtd_set_epsilon(const fdtd_grid *g, const void *eps, const void *sigma, int
 
 /* ---- diagnostics --------------------------------------------------------- */
 
-/* Device time of each launch of fdtd_step, for measurement.  enable != 0 clears
- * the sums and records CUDA events around every launch of each following
- * fdtd_step on its stream; enable == 0 stops recording.  fdtd_profile_read
- * waits for the recorded events and returns the summed milliseconds per
- * launch, [0] CPML-shell H on the side stream (concurrent with [2]), [1] the
- * shell E cells run on the side stream (none unless FDTD_B200_SHELL_SPLIT=1
- * selects that schedule), [2] the interior single-pass kernel, [3] the plane
- * DFT (of the interior cells, or with the face marches of the whole planes),
- * [4] the shell E cells after the join (the face marches and the per-cell
- * edges beside them, or the per-cell kernel with sources and DFTs), and the
- * number of steps recorded.  A step that runs as one march (fdtd_step_swap) has
- * it in [2]; [0], [1] and [4] are then empty.  No reference counterpart. */
+/* Device time of each launch of a fused step, for measurement.  enable != 0
+ * clears the sums and records CUDA events around every launch of each following
+ * fdtd_step and fdtd_step_swap on its stream; enable == 0 stops recording.
+ * fdtd_profile_read waits for the recorded events and returns the number of steps
+ * recorded and the summed milliseconds per launch.  With FDTD_SCHEDULE_INTERIOR
+ * and FDTD_SCHEDULE_FACES these are [0] CPML-shell H on the side stream
+ * (concurrent with [2]), [1] the shell E cells run on the side stream (none unless
+ * FDTD_B200_SHELL_SPLIT=1 selects that), [2] the interior single-pass kernel, [3]
+ * the plane DFT (of the interior cells, or with the face marches of the whole
+ * planes), [4] the shell E cells after the join (the face marches and the per-cell
+ * edges beside them, or the per-cell kernel with sources and DFTs).  With
+ * FDTD_SCHEDULE_MARCH [2] is the march and [3] the plane DFTs, with
+ * FDTD_SCHEDULE_GRID [0] the H launch and [4] the E launch with sources and DFTs;
+ * their other slots stay 0.  fdtd_profile_schedules returns how many of the steps
+ * recorded ran by each schedule.  No reference counterpart. */
 int fdtd_profile_steps(int32_t enable);
 int fdtd_profile_read(double ms[5], int32_t *nsteps);
+int fdtd_profile_schedules(int32_t steps[FDTD_SCHEDULES]);
 
 /* Number of kernel launches this library has issued since it was loaded. */
 int64_t fdtd_launch_count(void);

@@ -32,6 +32,11 @@ FDTD_SRC_EX = 1
 FDTD_N2F_BF16X3 = 0
 FDTD_N2F_TF32 = 1
 FDTD_N2F_FP64 = 2
+FDTD_SCHEDULE_MARCH = 0
+FDTD_SCHEDULE_GRID = 1
+FDTD_SCHEDULE_INTERIOR = 2
+FDTD_SCHEDULE_FACES = 3
+FDTD_SCHEDULES = 4
 FDTD_WAIT_INTERIOR = 0
 FDTD_WAIT_N2F = 1
 
@@ -108,6 +113,7 @@ SIGNATURES = {
                             c_int32, POINTER(PlaneDft), c_int32, c_void_p]),
     "fdtd_step_swap": (c_int32, [POINTER(Grid), POINTER(Fields), POINTER(Cpml), POINTER(Source),
                                  c_int32, POINTER(PlaneDft), c_int32, c_void_p]),
+    "fdtd_step_schedule": (c_int32, [POINTER(Grid), c_int32, POINTER(c_int32)]),
     "fdtd_add_source": (c_int32, [POINTER(Grid), c_void_p, c_void_p, POINTER(Source), c_void_p]),
     "fdtd_dft_faces": (c_int32, [POINTER(Grid), POINTER(c_void_p), POINTER(c_void_p),
                                  POINTER(Box), c_void_p, c_void_p, c_void_p]),
@@ -130,6 +136,7 @@ SIGNATURES = {
                                    c_double, POINTER(c_void_p), POINTER(c_void_p), c_void_p]),
     "fdtd_profile_steps": (c_int32, [c_int32]),
     "fdtd_profile_read": (c_int32, [POINTER(c_double), POINTER(c_int32)]),
+    "fdtd_profile_schedules": (c_int32, [POINTER(c_int32)]),
     "fdtd_launch_count": (c_int64, []),
     "fdtd_farfield_eh": (c_int32, [c_void_p, c_int32, c_void_p, c_int32, c_double, c_double,
                                    c_void_p, c_void_p]),

@@ -31,6 +31,7 @@ cudaError_t launch_farfield_eh(const void *nl, int nl_f64, const double *obs, in
                                double k_wave, double eta0, double *eh, cudaStream_t st);
 void profile_enable(bool on);
 cudaError_t profile_read(double ms[5], int *steps);
+void profile_schedules(int32_t steps[FDTD_SCHEDULES]);
 struct MatScalars {
     double scale, dt, two_eps0, eps0;
 };
@@ -505,6 +506,21 @@ int fdtd_step_swap(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
     return step_impl(g, f, c, src, nsrc, planes, nplanes, stream, true, "step_swap");
 }
 
+int fdtd_step_schedule(const fdtd_grid *g, int32_t swap, int32_t *schedule) {
+    int rc;
+    if ((rc = check_grid(g))) return rc;
+    if (!schedule) return fail(FDTD_ERR_INVALID, "NULL output");
+    fdtd_fields f;
+    fdtd_cpml c;
+    memset(&f, 0, sizeof(f));
+    memset(&c, 0, sizeof(c));
+    for (int q = 0; q < 6; ++q) c.psi_h_next[q] = (void *)(uintptr_t)256;  // apart, and aligned
+    *schedule = g->dtype == FDTD_F32
+                    ? fdtd::step_schedule<float>(make_args<float>(g, &f, &c, swap != 0))
+                    : fdtd::step_schedule<double>(make_args<double>(g, &f, &c, swap != 0));
+    return FDTD_OK;
+}
+
 int fdtd_add_source(const fdtd_grid *g, void *Ex, const void *ce_x, const fdtd_source *src,
                     void *stream) {
     int rc;
@@ -719,6 +735,12 @@ int fdtd_profile_read(double ms[5], int32_t *nsteps) {
     cudaError_t e = fdtd::profile_read(ms, &n);
     *nsteps = n;
     return cuda_status(e, "profile_read");
+}
+
+int fdtd_profile_schedules(int32_t steps[FDTD_SCHEDULES]) {
+    if (!steps) return fail(FDTD_ERR_INVALID, "NULL output");
+    fdtd::profile_schedules(steps);
+    return FDTD_OK;
 }
 
 int64_t fdtd_launch_count(void) { return fdtd::g_launches.load(std::memory_order_relaxed); }

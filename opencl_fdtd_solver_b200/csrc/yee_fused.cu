@@ -620,35 +620,42 @@ struct StepProfiler {
     std::mutex mu;
     bool on = false;
     std::vector<std::array<cudaEvent_t, NEV>> pending;
-    std::vector<bool> dft_last;  // per pending step: the plane DFT ran after shell E
+    std::vector<int> sched;  // schedule of each pending step
     double ms[NPROF] = {0.0, 0.0, 0.0, 0.0, 0.0};
     int steps = 0;
+    int by_sched[FDTD_SCHEDULES] = {0, 0, 0, 0};
 };
 StepProfiler g_prof;
 
 // Waits for the recorded steps, adds their launch times, releases the events.
 cudaError_t prof_flush_locked() {
     cudaError_t err = cudaSuccess;
+    // ev: 0 start, 1 shell H done (side stream), 2 outer shell E done (side),
+    // 3 interior or march done, 4 joined, 5 plane DFT done, 6 rim E done; with the
+    // face kernels 5 is shell E done and 6 plane DFT done
+    constexpr int SPAN[FDTD_SCHEDULES][NPROF][2] = {
+        {{-1, -1}, {-1, -1}, {0, 3}, {5, 6}, {-1, -1}},   // march, plane DFTs
+        {{0, 1}, {-1, -1}, {-1, -1}, {-1, -1}, {5, 6}},   // H, E
+        {{0, 1}, {1, 2}, {0, 3}, {4, 5}, {5, 6}},
+        {{0, 1}, {1, 2}, {0, 3}, {5, 6}, {4, 5}}};
     for (size_t q = 0; q < g_prof.pending.size(); ++q) {
         auto &ev = g_prof.pending[q];
-        // ev: 0 start, 1 shell H done (side stream), 2 outer shell E done (side),
-        // 3 interior done, 4 joined, 5 plane DFT done, 6 rim E done; with the
-        // face kernels 5 is shell E done and 6 plane DFT done
+        const int sched = g_prof.sched[q];
         cudaError_t e = cudaEventSynchronize(ev[6]);
-        const bool late = g_prof.dft_last[q];
-        const int from[NPROF] = {0, 1, 0, late ? 5 : 4, late ? 4 : 5};
-        const int to[NPROF] = {1, 2, 3, late ? 6 : 5, late ? 5 : 6};
         for (int s = 0; s < NPROF && e == cudaSuccess; ++s) {
+            const int from = SPAN[sched][s][0], to = SPAN[sched][s][1];
+            if (from < 0) continue;
             float t = 0.f;
-            e = cudaEventElapsedTime(&t, ev[from[s]], ev[to[s]]);
+            e = cudaEventElapsedTime(&t, ev[from], ev[to]);
             g_prof.ms[s] += t;
         }
         if (e != cudaSuccess) err = e;
         for (cudaEvent_t x : ev) cudaEventDestroy(x);
         ++g_prof.steps;
+        ++g_prof.by_sched[sched];
     }
     g_prof.pending.clear();
-    g_prof.dft_last.clear();
+    g_prof.sched.clear();
     return err;
 }
 
@@ -663,10 +670,10 @@ bool prof_begin(std::array<cudaEvent_t, NEV> &ev) {
     return true;
 }
 
-void prof_end(const std::array<cudaEvent_t, NEV> &ev, bool dft_last) {
+void prof_end(const std::array<cudaEvent_t, NEV> &ev, int sched) {
     std::lock_guard<std::mutex> lk(g_prof.mu);
     g_prof.pending.push_back(ev);
-    g_prof.dft_last.push_back(dft_last);
+    g_prof.sched.push_back(sched);
     if (g_prof.pending.size() >= 2048) prof_flush_locked();
 }
 }  // namespace
@@ -736,6 +743,7 @@ void profile_enable(bool on) {
     if (on) {
         prof_flush_locked();
         for (double &m : g_prof.ms) m = 0.0;
+        for (int &n : g_prof.by_sched) n = 0;
         g_prof.steps = 0;
     }
     g_prof.on = on;
@@ -747,6 +755,12 @@ cudaError_t profile_read(double ms[5], int *steps) {
     for (int s = 0; s < NPROF; ++s) ms[s] = g_prof.ms[s];
     *steps = g_prof.steps;
     return e;
+}
+
+void profile_schedules(int32_t steps[FDTD_SCHEDULES]) {
+    std::lock_guard<std::mutex> lk(g_prof.mu);
+    prof_flush_locked();
+    for (int s = 0; s < FDTD_SCHEDULES; ++s) steps[s] = g_prof.by_sched[s];
 }
 
 // FDTD_B200_SHELL_SPLIT=1 splits the shell E cells whose stencils read no H of
@@ -781,7 +795,7 @@ static cudaError_t launch_step_march(const YeeArgs<T> &a, const SourceList &src,
     if (e == cudaSuccess && pl.n) e = launch_plane_dft_box<T>(a, all, pl, st);
     if (prof) {
         cudaEventRecord(ev[6], st);
-        prof_end(ev, true);
+        prof_end(ev, FDTD_SCHEDULE_MARCH);
     }
     return e;
 }
@@ -802,7 +816,7 @@ static cudaError_t launch_step_grid(const YeeArgs<T> &a, const SourceList &src,
     if (e == cudaSuccess) e = launch_shell_E<T>(a, none, src, pl, st);
     if (prof) {
         cudaEventRecord(ev[6], st);
-        prof_end(ev, false);
+        prof_end(ev, FDTD_SCHEDULE_GRID);
     }
     return e;
 }
@@ -821,44 +835,72 @@ static cudaError_t launch_step_grid(const YeeArgs<T> &a, const SourceList &src,
 // waits of the interior march and its launch counts are tested on such a grid.
 constexpr int64_t GRID_MIN_CELLS = 100000;
 
+// Interior H box B = [npml, N-npml)^3 (x on a slab: [pml_lo, nx - pml_hi -
+// ghost_hi), so the upper ghost plane, whose forward differences would read past the
+// slab, is left to the boundary-guarded shell kernel).
 template <typename T>
-cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const PlaneList &pl,
-                              cudaStream_t st) {
-    const int elem = (int)sizeof(T);
+static void interior_box(const YeeArgs<T> &a, int blo[3], int bhi[3]) {
     const int n[3] = {a.nx, a.ny, a.nz};
-    if (face_mode() != 1 && march_path_ok<T>(a)) {
-        const cudaError_t e = launch_step_march<T>(a, src, pl, st);
-        if (e != cudaErrorNotSupported) return e;  // else no tensor maps, nothing launched
-    }
-    const int64_t cells = (int64_t)a.nx * a.ny * a.nz;
-    const bool swap = a.psi_h_next[0] != a.psi_h[0];
-    if (face_mode() != 1 && cells >= GRID_MIN_CELLS &&
-        (!march_size<T>(cells) ||
-         (!a.ghost_lo && !a.ghost_hi &&
-          (5 * a.npml >= a.nz || a.lossy ||
-           (swap && !interior_pays(a.nx, a.nz, a.npml, march_pad<T>(a.ny, a.nz)) &&
-            !interior_beats_grid<T>(a.nx, a.ny, a.nz, a.npml))))))
-        return launch_step_grid<T>(a, src, pl, st);
-    // interior H box B = [npml, N-npml)^3 (x on a slab: [pml_lo, nx - pml_hi -
-    // ghost_hi), so the upper ghost plane, whose forward differences would read
-    // past the slab, is left to the boundary-guarded shell kernel); the fused
-    // kernel needs npml >= 1, a box of at least two cells per axis and
-    // TMA-compatible (16-byte) strides and base addresses
-    int blo[3], bhi[3];
     for (int d = 0; d < 3; ++d) {
         blo[d] = a.npml;
         bhi[d] = n[d] - a.npml;
     }
     blo[0] = a.xb.pml_lo;
     bhi[0] = n[0] - a.xb.pml_hi - a.ghost_hi;
-    bool use_interior = a.npml >= 1 && ((int64_t)a.nz * elem) % 16 == 0;
-    for (int d = 0; d < 3; ++d) use_interior = use_interior && bhi[d] - blo[d] >= 2;
-    for (int c = 0; c < 3 && use_interior; ++c) {
+}
+
+// The interior kernel needs npml >= 1, a box of at least two cells per axis and
+// TMA-compatible (16-byte) strides and base addresses.
+template <typename T>
+static bool interior_path_ok(const YeeArgs<T> &a) {
+    int blo[3], bhi[3];
+    interior_box<T>(a, blo, bhi);
+    if (a.npml < 1 || ((int64_t)a.nz * (int64_t)sizeof(T)) % 16 != 0) return false;
+    for (int d = 0; d < 3; ++d)
+        if (bhi[d] - blo[d] < 2) return false;
+    for (int c = 0; c < 3; ++c) {
         const void *ptrs[5] = {a.E[c], a.H[c], a.ce[c], a.E_next[c], a.H_next[c]};
         for (const void *q : ptrs)
-            if (reinterpret_cast<uintptr_t>(q) % 16 != 0) use_interior = false;
-        if (a.lossy && reinterpret_cast<uintptr_t>(a.ca[c]) % 16 != 0) use_interior = false;
+            if (reinterpret_cast<uintptr_t>(q) % 16 != 0) return false;
+        if (a.lossy && reinterpret_cast<uintptr_t>(a.ca[c]) % 16 != 0) return false;
     }
+    return true;
+}
+
+template <typename T>
+int step_schedule(const YeeArgs<T> &a, bool march) {
+    const int64_t cells = (int64_t)a.nx * a.ny * a.nz;
+    if (face_mode() != 1) {
+        if (march && march_path_ok<T>(a)) return FDTD_SCHEDULE_MARCH;
+        const bool swap = a.psi_h_next[0] != a.psi_h[0];
+        if (cells >= GRID_MIN_CELLS &&
+            (!march_size<T>(cells) ||
+             (!a.ghost_lo && !a.ghost_hi &&
+              (5 * a.npml >= a.nz || a.lossy ||
+               (swap && !interior_pays(a.nx, a.nz, a.npml, march_pad<T>(a.ny, a.nz)) &&
+                !interior_beats_grid<T>(a.nx, a.ny, a.nz, a.npml))))))
+            return FDTD_SCHEDULE_GRID;
+    }
+    if (!interior_path_ok<T>(a)) return FDTD_SCHEDULE_GRID;
+    return !split_shell_e() && face_path_ok<T>(a) ? FDTD_SCHEDULE_FACES : FDTD_SCHEDULE_INTERIOR;
+}
+
+template int step_schedule<float>(const YeeArgs<float> &, bool);
+template int step_schedule<double>(const YeeArgs<double> &, bool);
+
+template <typename T>
+cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const PlaneList &pl,
+                              cudaStream_t st) {
+    int sched = step_schedule<T>(a);
+    if (sched == FDTD_SCHEDULE_MARCH) {
+        const cudaError_t e = launch_step_march<T>(a, src, pl, st);
+        if (e != cudaErrorNotSupported) return e;  // else no tensor maps, nothing launched
+        sched = step_schedule<T>(a, false);
+    }
+    if (sched == FDTD_SCHEDULE_GRID) return launch_step_grid<T>(a, src, pl, st);
+    const int n[3] = {a.nx, a.ny, a.nz};
+    int blo[3], bhi[3];
+    interior_box<T>(a, blo, bhi);
     // tile shape: the one that pads the interior's k extent [lo, hi) least
     // (k0 starts at lo rounded down to a 16-byte boundary)
     int gsel = 16;
@@ -871,9 +913,8 @@ cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const 
         if (5 * ((ext + w16 - 1) / w16 * w16) > 6 * ((ext + w8 - 1) / w8 * w8)) gsel = 8;
     }
     FusedMaps maps;
-    if (use_interior && !(gsel == 8 ? build_maps<T, 8>(a, maps) : build_maps<T, 16>(a, maps)))
-        use_interior = false;
-    if (!use_interior) return launch_step_grid<T>(a, src, pl, st);
+    if (!(gsel == 8 ? build_maps<T, 8>(a, maps) : build_maps<T, 16>(a, maps)))
+        return launch_step_grid<T>(a, src, pl, st);
     // hbox = B (H of the interior kernel), ebox = B' (its E), rbox = [lo, hi+1):
     // the E cells outside rbox read no H of B, the rim rbox \ B' does
     ShellBox hbox, ebox, rbox, all;
@@ -911,7 +952,7 @@ cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const 
     e2 = cudaStreamWaitEvent(st, side->join, 0);
     if (e == cudaSuccess) e = e2;
     if (prof) cudaEventRecord(ev[4], st);
-    bool faces = !split_shell_e() && face_path_ok<T>(a);
+    bool faces = sched == FDTD_SCHEDULE_FACES;
     if (faces && e == cudaSuccess) {
         // shell E through the CPML face marches, then the plane DFTs of every
         // monitored cell in one pass over the planes
@@ -935,7 +976,7 @@ cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const 
     }
     if (prof) {
         cudaEventRecord(ev[6], st);
-        prof_end(ev, faces);
+        prof_end(ev, faces ? FDTD_SCHEDULE_FACES : FDTD_SCHEDULE_INTERIOR);
     }
     return e;
 }

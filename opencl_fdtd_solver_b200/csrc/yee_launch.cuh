@@ -169,5 +169,9 @@ cudaError_t launch_add_source(int nx, int ny, int nz, const fdtd_source &s, T *E
 template <typename T>
 cudaError_t launch_step_fused(const YeeArgs<T> &a, const SourceList &src, const PlaneList &pl,
                               cudaStream_t st);
+// Which of the FDTD_SCHEDULE_* it takes for the arguments' grid and buffers.
+// march: the march may be taken; it may not once its tensor maps could not be built.
+template <typename T>
+int step_schedule(const YeeArgs<T> &a, bool march = true);
 
 }  // namespace fdtd
