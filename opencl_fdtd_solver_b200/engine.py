@@ -32,6 +32,7 @@ import contextlib
 import ctypes
 import logging
 import warnings
+from types import SimpleNamespace
 from typing import Sequence
 
 import numpy as np
@@ -168,16 +169,21 @@ class CUDAFDTD(SourceMonitorMixin):
 
     @staticmethod
     def device_footprint_bytes(shape, npml, dtype=np.float32, *, lossy=False, fused=True):
-        """Bytes this engine actually allocates: fields (twice when fused, the step
-        reads one set and writes the other), ``ce`` (and ``ca`` when lossy), ψ stripes."""
+        """Bytes this engine cannot do without: fields (twice when fused, the step
+        reads one set and writes the other), ``ce`` (and ``ca`` when lossy), ψ stripes.
+        The march's second ψ_H set comes on top where there is room for it."""
         nx, ny, nz = shape
         item = np.dtype(dtype).itemsize
         cells = nx * ny * nz
         arrays = 6 * (2 if fused else 1) + 3 + (3 if lossy else 0)
-        psi_one = 0
-        if npml > 0:
-            psi_one = 2 * (2 * npml * ny * nz + nx * 2 * npml * nz + nx * ny * 2 * npml)
-        return (arrays * cells + psi_one * 2) * item
+        return arrays * cells * item + 2 * CUDAFDTD._psi_set_bytes(shape, npml, dtype)
+
+    @staticmethod
+    def _psi_set_bytes(shape, npml, dtype):
+        """One of the ψ_H and ψ_E sets: two stripes along each axis."""
+        nx, ny, nz = shape
+        stripes = 2 * max(0, npml) * (ny * nz + nx * nz + nx * ny)
+        return 2 * stripes * np.dtype(dtype).itemsize
 
     @classmethod
     def device_memory_budget_bytes(cls, device):
@@ -191,10 +197,19 @@ class CUDAFDTD(SourceMonitorMixin):
         reserve = max(int(total * cls.MEMORY_HEADROOM_FRACTION), int(cls.MEMORY_HEADROOM_BYTES))
         return max(0, total - reserve)
 
+    @classmethod
+    def _second_psi_h_fits(cls, shape, npml, dtype, budget, free, total):
+        """Whether a second ψ_H set leaves the headroom whole: in the budget, and in the
+        ``free`` of the device's ``total`` bytes once the engine's own buffers are made."""
+        extra = cls._psi_set_bytes(shape, npml, dtype)
+        reserve = total - cls.device_memory_budget_bytes(SimpleNamespace(global_mem_size=total))
+        return (cls.device_footprint_bytes(shape, npml, dtype) + extra <= budget
+                and extra + reserve <= free)
+
     def _check_device_memory(self, shape, npml, dtype, device):
         needed = max(self.estimate_device_memory_bytes(shape, npml, dtype),
                      self.device_footprint_bytes(shape, npml, dtype, fused=self._fused_enabled))
-        budget = self.device_memory_budget_bytes(device)
+        self._memory_budget = budget = self.device_memory_budget_bytes(device)
         if needed > budget:
             total = int(getattr(device, "global_mem_size", getattr(device, "total_memory", 0)))
             name = getattr(device, "name", "device")
@@ -257,16 +272,40 @@ class CUDAFDTD(SourceMonitorMixin):
         with torch.cuda.stream(self.queue):
             self._psi_h = stripes()
             self._psi_e = stripes()
-            # the fused step's second ψ_H set (``fdtd_step_swap``); a grid that fills
-            # the device does without it and steps through ``fdtd_step``
             self._psi_hn = None
-            if self._fused_enabled and n > 0:
+            if self._second_psi_h_pays():
                 try:
                     self._psi_hn = stripes()
                 except torch.OutOfMemoryError:
                     log.info("no memory for a second psi_H set; stepping with psi_H in place")
 
-    def _build_structs(self):
+    def _second_psi_h_pays(self):
+        """Whether a second ψ_H set (``fdtd_step_swap``) changes the grid's schedule, in
+        lossless or lossy media, and there is room for it.  Without it the engine steps
+        through ``fdtd_step``, with the same fields."""
+        if not self._fused_enabled or self.npml == 0:
+            return False
+        g = self._grid_struct()
+        out = ctypes.c_int32()
+
+        def schedule(lossy, swap):
+            g.lossy = lossy
+            capi.run("fdtd_step_schedule", g, swap, ctypes.byref(out))
+            return out.value
+
+        if all(schedule(lossy, 1) == schedule(lossy, 0) for lossy in (0, 1)):
+            return False
+        torch = _torch()
+        free, total = torch.cuda.mem_get_info(self.device)
+
+        def fits(free):
+            return self._second_psi_h_fits((self.Nx, self.Ny, self.Nz), self.npml, self.dtype,
+                                           self._memory_budget, free, total)
+
+        return fits(free) or fits(free + torch.cuda.memory_reserved(self.device)
+                                  - torch.cuda.memory_allocated(self.device))
+
+    def _grid_struct(self):
         g = capi.Grid()
         g.nx, g.ny, g.nz, g.npml = self.Nx, self.Ny, self.Nz, self.npml
         g.dtype = capi.FDTD_F32 if self.dtype == np.float32 else capi.FDTD_F64
@@ -278,7 +317,10 @@ class CUDAFDTD(SourceMonitorMixin):
         g.dtm = self.dt / MU0
         g.dtm_dl = self.dt / (MU0 * self.dl)
         g.inv_dl = 1.0 / self.dl
-        self._grid = g
+        return g
+
+    def _build_structs(self):
+        self._grid = self._grid_struct()
         cp = capi.Cpml()
         for a in range(3):
             for stag, (bn, cn, kn) in (("h", ("b_h", "c_h", "ik_h")), ("e", ("b_e", "c_e", "ik_e"))):
@@ -343,12 +385,26 @@ class CUDAFDTD(SourceMonitorMixin):
         narrow = eps.dtype == np.float32 and (sig is None or sig.dtype == np.float32)
         src = np.float32 if narrow else np.float64
         with torch.cuda.stream(self.queue):
-            eps_d = torch.from_numpy(np.ascontiguousarray(eps, dtype=src)).to(self.device)
-            sig_d = None
-            if sig is not None:
-                sig_d = torch.from_numpy(np.ascontiguousarray(sig, dtype=src)).to(self.device)
-                if self._ca is None:
-                    self._ca = [torch.empty_like(c) for c in self._ce]
+            def buffers():
+                up = lambda a: torch.from_numpy(  # noqa: E731
+                    np.ascontiguousarray(a, dtype=src)).to(self.device)
+                eps_d = up(eps)
+                if sig is None:
+                    return eps_d, None, None
+                return eps_d, up(sig), self._ca or [torch.empty_like(c) for c in self._ce]
+
+            try:
+                eps_d, sig_d, ca_t = buffers()
+            except torch.OutOfMemoryError:
+                if sig is None or self._psi_hn is None:
+                    raise
+                log.info("second psi_H set given up for ca; stepping with psi_H in place")
+                self._psi_hn = None
+                eps_d = None
+            if eps_d is None:  # outside the handler, which still holds what was allocated
+                eps_d, sig_d, ca_t = buffers()
+            if sig_d is not None:
+                self._ca = ca_t
             ce = (ctypes.c_void_p * 3)(*[c.data_ptr() for c in self._ce])
             ca = (ctypes.c_void_p * 3)(*([c.data_ptr() for c in self._ca] if sig_d is not None
                                          else [None, None, None]))
