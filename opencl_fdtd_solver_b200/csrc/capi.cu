@@ -832,7 +832,10 @@ int fdtd_n2f_contract(const fdtd_n2f_face *faces, int32_t nfaces, int32_t cur_dt
     P.partial = (float2 *)(ws + pl.partial_off);
     if ((e = fdtd::n2f::launch_contract(mode, P, nfreq, st)) != cudaSuccess)
         return cuda_status(e, "n2f_contract");
-    return cuda_status(fdtd::n2f::launch_combine(P, nfreq, (float2 *)nl, st), "n2f_combine");
+    e = cur_dtype == FDTD_F32
+            ? fdtd::n2f::launch_combine<float2>(mode, P, nfreq, (float2 *)nl, st)
+            : fdtd::n2f::launch_combine<double2>(mode, P, nfreq, (float2 *)nl, st);
+    return cuda_status(e, "n2f_combine");
 }
 
 int fdtd_farfield_eh(const void *nl, int32_t nl_dtype, const double *obs_xyz, int32_t n_obs,

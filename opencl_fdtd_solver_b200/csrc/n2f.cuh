@@ -43,7 +43,8 @@ template <typename CT>
 cudaError_t launch_pack(int mode, const Params &P, int nfreq, unsigned char *dst,
                         cudaStream_t st);
 cudaError_t launch_contract(int mode, const Params &P, int nfreq, cudaStream_t st);
-cudaError_t launch_combine(const Params &P, int nfreq, float2 *nl, cudaStream_t st);
+template <typename CT>
+cudaError_t launch_combine(int mode, const Params &P, int nfreq, float2 *nl, cudaStream_t st);
 template <typename CT>
 cudaError_t launch_fp64(const Params &P, int nfreq, double2 *nl, cudaStream_t st);
 int read_error(int reset);

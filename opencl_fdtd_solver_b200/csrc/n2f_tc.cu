@@ -862,23 +862,75 @@ __global__ void k_n2f_pack(Params P, int nfreq, unsigned char *ws) {
     }
 }
 
-// NL[f][o][6] (complex64) = Σ_faces partial[f][face][o][c] mapped to (J_b, J_c, M_b, M_c).
-__global__ void k_n2f_combine(Params P, int nfreq, float2 *nl) {
+// NL[o][6] of one frequency: Σ_faces partial[face][o][c] mapped to (J_b, J_c, M_b, M_c);
+// false if one of them is not finite.
+__device__ __forceinline__ bool combine_faces(const Params &P, int fr, int o, float2 *nl) {
+    float2 acc[6];
+    for (int c = 0; c < 6; ++c) acc[c] = make_float2(0.f, 0.f);
+    for (int fi = 0; fi < P.nfaces; ++fi) {
+        const float2 *p = P.partial + (((int64_t)fr * P.nfaces + fi) * P.n_obs + o) * 4;
+        for (int c = 0; c < 4; ++c) {
+            const int m = P.comp_map[fi * 4 + c];
+            acc[m].x += p[c].x;
+            acc[m].y += p[c].y;
+        }
+    }
+    bool ok = true;
+    for (int c = 0; c < 6; ++c) {
+        nl[c] = acc[c];
+        ok = ok && isfinite(acc[c].x) && isfinite(acc[c].y);
+    }
+    return ok;
+}
+
+// The same with the faces whose sums are not finite summed again in float64, straight
+// from the currents and with the phases rotated along a row.  A face with a current that
+// is not finite keeps its sums.
+template <typename CT>
+__device__ __noinline__ void combine_again(const Params &P, int fr, int o, float2 *nl) {
+    const double freq = P.freqs[fr];
+    for (int fi = 0; fi < P.nfaces; ++fi) {
+        float2 *out = P.partial + (((int64_t)fr * P.nfaces + fi) * P.n_obs + o) * 4;
+        bool ok = true;
+        for (int c = 0; c < 4; ++c) ok = ok && isfinite(out[c].x) && isfinite(out[c].y);
+        if (ok) continue;
+        const Face &F = P.face[fi];
+        const CT *cur = reinterpret_cast<const CT *>(P.cur[fi]) + (int64_t)fr * F.np * F.nq * 4;
+        const double rn = P.dirs[3 * o + F.axis_n], rp = P.dirs[3 * o + F.axis_p],
+                     rq = P.dirs[3 * o + F.axis_q];
+        const double base = rn * F.x_n + rp * F.o_p + rq * F.o_q;
+        const double2 W = zphase_turns(freq * F.pitch * rq / C0, 1.0);
+        double2 S[4] = {};
+        ok = true;
+        for (int p = 0; p < F.np && ok; ++p) {
+            double2 u = zphase_turns(freq * (base + rp * F.pitch * p) / C0, 1.0);
+            for (int q = 0; q < F.nq && ok; ++q, cur += 4) {
+                for (int c = 0; c < 4; ++c) {
+                    const double2 z = make_double2((double)cur[c].x, (double)cur[c].y);
+                    ok = ok && isfinite(z.x) && isfinite(z.y);
+                    S[c].x += u.x * z.x - u.y * z.y;
+                    S[c].y += u.x * z.y + u.y * z.x;
+                }
+                u = zmul(u, W);
+            }
+        }
+        for (int c = 0; c < 4 && ok; ++c) out[c] = make_float2((float)S[c].x, (float)S[c].y);
+    }
+    combine_faces(P, fr, o, nl);
+}
+
+// AGAIN (the folded sums): the sums of up to four currents leave float32 (and bfloat16)
+// where the currents themselves, from 8.5e37 on, and their far field do not.  A direction
+// that comes out infinite or NaN is therefore summed again directly; the check of the
+// results costs the others nothing measurable.
+template <typename CT, bool AGAIN>
+__global__ void k_n2f_combine(const __grid_constant__ Params P, int nfreq, float2 *nl) {
     const int64_t n = (int64_t)nfreq * P.n_obs;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
          q += (int64_t)gridDim.x * blockDim.x) {
         const int fr = (int)(q / P.n_obs), o = (int)(q % P.n_obs);
-        float2 acc[6];
-        for (int c = 0; c < 6; ++c) acc[c] = make_float2(0.f, 0.f);
-        for (int fi = 0; fi < P.nfaces; ++fi) {
-            const float2 *p = P.partial + (((int64_t)fr * P.nfaces + fi) * P.n_obs + o) * 4;
-            for (int c = 0; c < 4; ++c) {
-                const int m = P.comp_map[fi * 4 + c];
-                acc[m].x += p[c].x;
-                acc[m].y += p[c].y;
-            }
-        }
-        for (int c = 0; c < 6; ++c) nl[q * 6 + c] = acc[c];
+        const bool ok = combine_faces(P, fr, o, nl + q * 6);
+        if (AGAIN && !ok) combine_again<CT>(P, fr, o, nl + q * 6);
     }
 }
 
@@ -1044,11 +1096,15 @@ cudaError_t launch_contract(int mode, const Params &Pin, int nfreq, cudaStream_t
                : launch_tc<FDTD_N2F_TF32, false>(P, nfreq, st);
 }
 
-cudaError_t launch_combine(const Params &P, int nfreq, float2 *nl, cudaStream_t st) {
+template <typename CT>
+cudaError_t launch_combine(int mode, const Params &P, int nfreq, float2 *nl, cudaStream_t st) {
     const int64_t n = (int64_t)nfreq * P.n_obs;
     int64_t blocks = (n + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    k_n2f_combine<<<(unsigned)blocks, 256, 0, st>>>(P, nfreq, nl);
+    if (folded(mode))
+        k_n2f_combine<CT, true><<<(unsigned)blocks, 256, 0, st>>>(P, nfreq, nl);
+    else
+        k_n2f_combine<CT, false><<<(unsigned)blocks, 256, 0, st>>>(P, nfreq, nl);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -1073,6 +1129,8 @@ int read_error(int reset) {
 
 template cudaError_t launch_pack<float2>(int, const Params &, int, unsigned char *, cudaStream_t);
 template cudaError_t launch_pack<double2>(int, const Params &, int, unsigned char *, cudaStream_t);
+template cudaError_t launch_combine<float2>(int, const Params &, int, float2 *, cudaStream_t);
+template cudaError_t launch_combine<double2>(int, const Params &, int, float2 *, cudaStream_t);
 template cudaError_t launch_fp64<float2>(const Params &, int, double2 *, cudaStream_t);
 template cudaError_t launch_fp64<double2>(const Params &, int, double2 *, cudaStream_t);
 
