@@ -781,7 +781,13 @@ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // Chunks along x.  A CTA costs its planes plus about two and a half (pipeline
 // fill, the H-only plane before and the E-only plane after), an x-CPML plane
 // about 1.6 middle ones.  CTAs that fit the slots (two per SM) run as one wave of
-// the longest; more run at the mean load plus about half a chunk of tail.
+// the longest, which lies in a y or z slab and takes about 1.6 middle ones a plane
+// too; more, the costliest first, run at the mean load plus about half a chunk of
+// tail.  (Without the 1.6, grids of 1 to 4 M cells got one wave of long chunks, slower
+// than the schedules that the march replaces: FP64 112³ npml 8 74.2 us a step against
+// 54.5 now, 56 by two whole-grid launches and 53 by the interior march; 314x56x144 npml 4
+// 108 / 82 / 90 / 88; FP32 252x197x56 npml 3 85 / 62 / 61 / 72, 404x62x184 npml 4 98 / 82 /
+// 88 / 82, 270x46x392 npml 4 116 / 89 / 89 / 84.)
 void march_chunks(MarchBox &bx, int P, int mid) {
     const int slots = 2 * device_sm_count();
     double best = 1e30;
@@ -795,7 +801,7 @@ void march_chunks(MarchBox &bx, int P, int mid) {
         const double cx = 1.6 * (xlen + 2.5), cm = len + 2.5;
         const double load = bx.tiles * (nm * cm + nx2 * cx) / slots;
         const double longest = cx > cm ? cx : cm;
-        const double est = bx.tiles * (nm + nx2) <= slots ? longest : load + 0.5 * longest;
+        const double est = bx.tiles * (nm + nx2) <= slots ? 1.6 * longest : load + 0.5 * longest;
         if (est < best - 1e-9) {
             best = est;
             bx.chunk = len;
