@@ -99,15 +99,26 @@ inline bool interior_pays(int nx, int nz, int npml, double pad) {
     return pad > 1.05 && nz >= 20 * npml && (nx <= 256 || pad > 1.2);
 }
 
-// And those, not for the march, with long rows, enough cells and little CPML: FP32,
-// interior march / two whole-grid launches, 84x296x264 npml 10 120 / 129, 62x200x352 npml
-// 8 82.6 / 86.8, 328x224x208 npml 8 234 / 266; but 150x136x176 npml 10 78.6 / 74.7,
-// 280x216x80 npml 6 127 / 99, 192³ npml 20 157 / 149.
+// Padding of the interior box's (j, k) extent to the interior march's 64 x 8 (FP64: 32 x
+// 8) tiles, which start on a 16-byte boundary.
+template <typename T>
+inline double interior_pad(int ny, int nz, int npml) {
+    constexpr int V = 16 / (int)sizeof(T);
+    return tile_pad(ny - 2 * npml, nz - npml - npml / V * V, 256 / (int)sizeof(T), 8);
+}
+
+// And those, not for the march, with long rows, enough cells and little CPML, or whose
+// interior box fits the tiles: FP32, interior march / two whole-grid launches, 84x296x264
+// npml 10 119.7 / 128.0, 62x200x352 npml 8 82.0 / 86.1, 328x224x208 npml 8 232 / 265, 144³
+// npml 8 58.2 / 63.7, 192x162x144 npml 10 91.3 / 93.4; but 280x216x80 npml
+// 6 126 / 99, 160x160x96 npml 12 64.5 / 57.7.
 template <typename T>
 inline bool interior_beats_grid(int nx, int ny, int nz, int npml) {
     const int64_t cells = (int64_t)nx * ny * nz;
-    return nz * (int)sizeof(T) >= 768 && cells * (int)sizeof(T) >= 16000000 &&
-           pml_fraction(nx, ny, nz, npml) <= 0.42;
+    const double f = pml_fraction(nx, ny, nz, npml);
+    const int row = nz * (int)sizeof(T);
+    return (row >= 768 && cells * (int)sizeof(T) >= 16000000 && f <= 0.42) ||
+           (row >= 512 && f <= 0.4 && interior_pad<T>(ny, nz, npml) < 1.1);
 }
 
 // Where the march beats the two whole-grid launches.  Its CPML tiles evaluate their

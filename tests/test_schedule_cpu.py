@@ -30,6 +30,8 @@ def schedule(shape, npml, f64, lossy, swap, slab=None):
     ((160, 160, 96), 12, 0, 0, GRID, INTERIOR),         # narrow tile
     ((72, 224, 328), 4, 0, 0, INTERIOR, INTERIOR),      # padded, few planes
     ((64, 64, 64), 8, 0, 0, GRID, GRID),                # fits the L2
+    ((144, 144, 144), 8, 0, 0, INTERIOR, INTERIOR),     # whole tiles in the interior
+    ((118, 448, 152), 16, 0, 0, GRID, INTERIOR),
     ((40, 36, 48), 6, 0, 0, INTERIOR, INTERIOR),
     ((37, 41, 53), 6, 0, 1, GRID, GRID),                # odd rows
     ((181, 230, 155), 10, 0, 0, GRID, GRID),
