@@ -345,12 +345,13 @@ def run_steps_timed(g, k):
     capi.run("fdtd_profile_schedules", by_sched)
     # the profile's slots, by the schedule that the steps took (none: split kernels)
     slots = {capi.FDTD_SCHEDULE_MARCH: {2: "k_march", 3: "k_plane_dft_box"},
-             capi.FDTD_SCHEDULE_GRID: {0: "k_shell_H", 4: "k_shell_E"}}
+             capi.FDTD_SCHEDULE_GRID: {0: "k_shell_H", 4: "k_shell_E", 3: "k_plane_dft_box"}}
     interior = dict(enumerate(("k_shell_H", "k_shell_E_side", "k_interior", "k_plane_dft_box",
                                "k_shell_E")))
     sched = max(range(capi.FDTD_SCHEDULES), key=lambda s: by_sched[s])
     per_kernel = {name: ms[i] / nsteps.value
-                  for i, name in slots.get(sched, interior).items()} if nsteps.value else {}
+                  for i, name in slots.get(sched, interior).items()
+                  if ms[i] or sched not in slots} if nsteps.value else {}
     phases = {f"ms_per_step_first_{split}": round(start.elapsed_time(mid) / max(1, split), 4)}
     if k > split:
         phases[f"ms_per_step_after_{split}"] = round(mid.elapsed_time(end) / (k - split), 4)
@@ -395,8 +396,8 @@ def run_b200_arm(args, rank, world, local):
         k_bytes = interior_alg_bytes(shape, npml, item)
         kname = "k_interior"
     else:
-        # two launches over the whole grid, the plane DFT in the second
-        kname = "k_shell_H + k_shell_E" if per_kernel else "step (split kernels)"
+        # two launches over the whole grid, the plane DFT in the second or after it
+        kname = " + ".join(per_kernel) if per_kernel else "step (split kernels)"
         k_ms, k_bytes = sum(per_kernel.values()) or ms_per_step, bpc * cells
     achieved = k_bytes / (k_ms / 1e3) / 1e9
     traffic = None

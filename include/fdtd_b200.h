@@ -155,7 +155,7 @@ int fdtd_step_swap(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
                    const fdtd_plane_dft *planes, int32_t nplanes, void *stream);
 
 /* How a fused step runs: one march over every cell, then the plane DFTs; two
- * launches over every cell (H, then E with the DFTs fused); the interior march
+ * launches over every cell (H, then E with most DFTs fused); the interior march
  * beside per-cell kernels for the CPML shell; the same with the shell's E by the
  * CPML face marches.  fdtd_step_schedule tells which one fdtd_step (swap == 0) or
  * fdtd_step_swap (swap != 0) takes for a grid whose buffers lie on 16-byte
@@ -398,8 +398,8 @@ int fdtd_set_epsilon(const fdtd_grid *g, const void *eps, const void *sigma, int
  * planes), [4] the shell E cells after the join (the face marches and the per-cell
  * edges beside them, or the per-cell kernel with sources and DFTs).  With
  * FDTD_SCHEDULE_MARCH [2] is the march and [3] the plane DFTs, with
- * FDTD_SCHEDULE_GRID [0] the H launch and [4] the E launch with sources and DFTs;
- * their other slots stay 0.  fdtd_profile_schedules returns how many of the steps
+ * FDTD_SCHEDULE_GRID [0] the H launch, [4] the E launch with sources and DFTs and [3]
+ * the DFTs of large z planes after it, if any; their other slots stay 0.  fdtd_profile_schedules returns how many of the steps
  * recorded ran by each schedule.  No reference counterpart. */
 int fdtd_profile_steps(int32_t enable);
 int fdtd_profile_read(double ms[5], int32_t *nsteps);

@@ -616,6 +616,7 @@ cudaError_t launch_interior(const YeeArgs<T> &a, const FusedMaps &maps, const Sh
 namespace {
 constexpr int NEV = 7;
 constexpr int NPROF = 5;
+constexpr int GRID_AND_DFT = FDTD_SCHEDULES;  // FDTD_SCHEDULE_GRID with z-plane DFTs after it
 struct StepProfiler {
     std::mutex mu;
     bool on = false;
@@ -633,11 +634,12 @@ cudaError_t prof_flush_locked() {
     // ev: 0 start, 1 shell H done (side stream), 2 outer shell E done (side),
     // 3 interior or march done, 4 joined, 5 plane DFT done, 6 rim E done; with the
     // face kernels 5 is shell E done and 6 plane DFT done
-    constexpr int SPAN[FDTD_SCHEDULES][NPROF][2] = {
+    constexpr int SPAN[FDTD_SCHEDULES + 1][NPROF][2] = {
         {{-1, -1}, {-1, -1}, {0, 3}, {5, 6}, {-1, -1}},   // march, plane DFTs
-        {{0, 1}, {-1, -1}, {-1, -1}, {-1, -1}, {5, 6}},   // H, E
+        {{0, 1}, {-1, -1}, {-1, -1}, {-1, -1}, {4, 5}},   // H, E
         {{0, 1}, {1, 2}, {0, 3}, {4, 5}, {5, 6}},
-        {{0, 1}, {1, 2}, {0, 3}, {5, 6}, {4, 5}}};
+        {{0, 1}, {1, 2}, {0, 3}, {5, 6}, {4, 5}},
+        {{0, 1}, {-1, -1}, {-1, -1}, {5, 6}, {4, 5}}};    // H, E, z-plane DFTs
     for (size_t q = 0; q < g_prof.pending.size(); ++q) {
         auto &ev = g_prof.pending[q];
         const int sched = g_prof.sched[q];
@@ -652,7 +654,7 @@ cudaError_t prof_flush_locked() {
         if (e != cudaSuccess) err = e;
         for (cudaEvent_t x : ev) cudaEventDestroy(x);
         ++g_prof.steps;
-        ++g_prof.by_sched[sched];
+        ++g_prof.by_sched[sched == GRID_AND_DFT ? FDTD_SCHEDULE_GRID : sched];
     }
     g_prof.pending.clear();
     g_prof.sched.clear();
@@ -800,11 +802,31 @@ static cudaError_t launch_step_march(const YeeArgs<T> &a, const SourceList &src,
     return e;
 }
 
+// The E launch over the whole grid accumulates plane DFTs with the cells.  A z plane has
+// one cell in each row, whose lane runs through the frequencies while its warp waits, so
+// from this many cells, and cells x frequencies, on it gets a pass over the plane after
+// the E launch (one more launch for the host, too).  Per step in us, with the E launch / after it, 1, 4, 8 and 16 frequencies:
+// FP32 48³ 9.7 / 10.5, 10.2 / 11.6, 11.6 / 12.8, 14.6 / 15.1; 64³ 12.8 / 13.1, 14.5 / 14.0,
+// 16.9 / 15.2, 21.5 / 17.2; 128³ 49.6 / 49.2, 59.5 / 51.1, 72.8 / 53.3, 99.7 / 57.4; FP64
+// 200x200x64 110.5 / 100.7, 129.5 / 102.6, 155.3 / 105.0, 202.7 / 110.1.  x and y planes,
+// whose cells are whole rows, gain nothing (128³, 16: x 48.9 / 57.4, y 57.1 / 57.1).
+constexpr int64_t Z_DFT_CELLS = 4000, Z_DFT_WORK = 30000;
+
 // The step as two launches over the whole grid, one thread per cell (yee_shell.cu
-// with an empty inner box), plane DFTs fused.
+// with an empty inner box), plane DFTs fused but for those of large z planes.
 template <typename T>
 static cudaError_t launch_step_grid(const YeeArgs<T> &a, const SourceList &src,
                                     const PlaneList &pl, cudaStream_t st) {
+    PlaneList with, after;
+    memset(&with, 0, sizeof(with));
+    memset(&after, 0, sizeof(after));
+    const int64_t zcells = (int64_t)a.nx * a.ny;
+    for (int q = 0; q < pl.n; ++q) {
+        const bool z = pl.p[q].axis == 2 && zcells >= Z_DFT_CELLS &&
+                       zcells * pl.p[q].nfreq >= Z_DFT_WORK;
+        PlaneList &l = z ? after : with;
+        l.p[l.n++] = pl.p[q];
+    }
     std::array<cudaEvent_t, NEV> ev;
     const bool prof = prof_begin(ev);
     if (prof) cudaEventRecord(ev[0], st);
@@ -812,11 +834,14 @@ static cudaError_t launch_step_grid(const YeeArgs<T> &a, const SourceList &src,
     memset(&none, 0, sizeof(none));
     cudaError_t e = launch_shell_H<T>(a, none, st);
     if (prof)
-        for (int s = 1; s < 6; ++s) cudaEventRecord(ev[s], st);
-    if (e == cudaSuccess) e = launch_shell_E<T>(a, none, src, pl, st);
+        for (int s = 1; s < 5; ++s) cudaEventRecord(ev[s], st);
+    if (e == cudaSuccess) e = launch_shell_E<T>(a, none, src, with, st);
+    if (prof) cudaEventRecord(ev[5], st);
+    const ShellBox all = whole_grid(a.nx, a.ny, a.nz);
+    if (e == cudaSuccess && after.n) e = launch_plane_dft_box<T>(a, all, after, st);
     if (prof) {
         cudaEventRecord(ev[6], st);
-        prof_end(ev, FDTD_SCHEDULE_GRID);
+        prof_end(ev, after.n ? GRID_AND_DFT : FDTD_SCHEDULE_GRID);
     }
     return e;
 }

@@ -26,18 +26,19 @@ def profile(g, n):
     return list(ms), list(sched)
 
 
-@pytest.mark.parametrize("shape,npml,schedule,filled", [
-    ((64, 64, 64), 8, "GRID", (0, 4)), ((37, 41, 53), 6, "GRID", (0, 4)),
-    ((192, 160, 192), 8, "MARCH", (2, 3)), ((40, 36, 48), 6, "INTERIOR", (0, 2, 3, 4)),
+@pytest.mark.parametrize("shape,npml,nfreq,schedule,filled", [
+    ((64, 64, 64), 8, 1, "GRID", (0, 4)), ((37, 41, 53), 6, 1, "GRID", (0, 4)),
+    ((64, 64, 64), 8, 8, "GRID", (0, 3, 4)),  # a z plane's DFTs after the E launch
+    ((192, 160, 192), 8, 1, "MARCH", (2, 3)), ((40, 36, 48), 6, 1, "INTERIOR", (0, 2, 3, 4)),
 ])
-def test_profile_slots_of_each_schedule(shape, npml, schedule, filled, monkeypatch):
+def test_profile_slots_of_each_schedule(shape, npml, nfreq, schedule, filled, monkeypatch):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from opencl_fdtd_solver_b200 import CUDAFDTD, CUDAPlaneDFTMonitor, _capi as capi
 
     monkeypatch.delenv("FDTD_B200_FACE_E", raising=False)
     g = CUDAFDTD(shape, 1e-3, npml=npml, dtype=np.float32)
-    CUDAPlaneDFTMonitor(g, 2, shape[2] // 2, [30e9])
+    CUDAPlaneDFTMonitor(g, 2, shape[2] // 2, [30e9 + 1e9 * q for q in range(nfreq)])
     g.run(2)
     ms, sched = profile(g, 5)
     assert sched[getattr(capi, "FDTD_SCHEDULE_" + schedule)] == 5
