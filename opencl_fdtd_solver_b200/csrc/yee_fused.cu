@@ -805,12 +805,14 @@ static cudaError_t launch_step_march(const YeeArgs<T> &a, const SourceList &src,
 // The E launch over the whole grid accumulates plane DFTs with the cells.  A z plane has
 // one cell in each row, whose lane runs through the frequencies while its warp waits, so
 // from this many cells, and cells x frequencies, on it gets a pass over the plane after
-// the E launch (one more launch for the host, too).  Per step in us, with the E launch / after it, 1, 4, 8 and 16 frequencies:
-// FP32 48³ 9.7 / 10.5, 10.2 / 11.6, 11.6 / 12.8, 14.6 / 15.1; 64³ 12.8 / 13.1, 14.5 / 14.0,
-// 16.9 / 15.2, 21.5 / 17.2; 128³ 49.6 / 49.2, 59.5 / 51.1, 72.8 / 53.3, 99.7 / 57.4; FP64
-// 200x200x64 110.5 / 100.7, 129.5 / 102.6, 155.3 / 105.0, 202.7 / 110.1.  x and y planes,
-// whose cells are whole rows, gain nothing (128³, 16: x 48.9 / 57.4, y 57.1 / 57.1).
-constexpr int64_t Z_DFT_CELLS = 4000, Z_DFT_WORK = 30000;
+// the E launch (one more launch for the host, too).  Per step in us, with the E launch /
+// after it, 1, 4, 8 and 16 frequencies: FP32 48³ 9.7 / 10.5, 10.2 / 11.6, 11.6 / 12.8, 14.6 /
+// 15.1; 96³ 22.3 / 22.9, 25.8 / 23.9, 30.5 / 25.5, 40.1 / 27.6; 128³ 49.6 / 49.2, 59.5 /
+// 51.1, 72.8 / 53.3, 99.7 / 57.4; FP64 200x200x64 110.5 / 100.7, 129.5 / 102.6, 155.3 / 105.0,
+// 202.7 / 110.1.  In smaller planes the lanes of several monitors wait side by side: 64³
+// with 8 frequencies 16.9 / 15.2, but with two z, an x and a y plane 21.5 / 24.0.  x and y
+// planes, whose cells are whole rows, gain nothing (128³, 16: x 48.9 / 57.4, y 57.1 / 57.1).
+constexpr int64_t Z_DFT_CELLS = 9000, Z_DFT_WORK = 30000;
 
 // The step as two launches over the whole grid, one thread per cell (yee_shell.cu
 // with an empty inner box), plane DFTs fused but for those of large z planes.

@@ -28,7 +28,7 @@ def profile(g, n):
 
 @pytest.mark.parametrize("shape,npml,nfreq,schedule,filled", [
     ((64, 64, 64), 8, 1, "GRID", (0, 4)), ((37, 41, 53), 6, 1, "GRID", (0, 4)),
-    ((64, 64, 64), 8, 8, "GRID", (0, 3, 4)),  # a z plane's DFTs after the E launch
+    ((96, 96, 62), 8, 4, "GRID", (0, 3, 4)),  # a z plane's DFTs after the E launch
     ((192, 160, 192), 8, 1, "MARCH", (2, 3)), ((40, 36, 48), 6, 1, "INTERIOR", (0, 2, 3, 4)),
 ])
 def test_profile_slots_of_each_schedule(shape, npml, nfreq, schedule, filled, monkeypatch):

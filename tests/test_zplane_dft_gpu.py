@@ -1,6 +1,6 @@
 """Plane DFTs of the two whole-grid launches against the CPU oracle, bit for bit (GPU).
 
-z planes on both sides of the two lines (4,000 cells, 30,000 cells x frequencies) above
+z planes on both sides of the two lines (9,000 cells, 30,000 cells x frequencies) above
 which they are accumulated in a pass of their own, in the first, a CPML, an inner and the
 last layer, next to x and y planes that stay with the E launch; up to the four planes that
 an engine takes.
@@ -22,9 +22,9 @@ torch = pytest.importorskip("torch")
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("shape,nfreqs", [
-    ((61, 67, 33), (7, 8, 16)),     # 4,087 cells: below, above the second line, well above
-    ((57, 70, 45), (8, 9, 17)),     # 3,990 cells: all with the E launch
-    ((60, 100, 35), (5, 4, 1)),     # 30,000 products, below, below
+    ((90, 100, 33), (3, 4, 16)),    # 9,000 cells: below, above the second line, well above
+    ((89, 101, 45), (4, 5, 17)),    # 8,989 cells: all with the E launch
+    ((100, 100, 35), (3, 2, 1)),    # 30,000 products, below, below
 ])
 def test_z_planes_vs_oracle(shape, nfreqs, dtype):
     if not torch.cuda.is_available():
