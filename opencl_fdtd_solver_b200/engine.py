@@ -295,12 +295,16 @@ class CUDAFDTD(SourceMonitorMixin):
 
         if all(schedule(lossy, 1) == schedule(lossy, 0) for lossy in (0, 1)):
             return False
+        shape = (self.Nx, self.Ny, self.Nz)
+        own = self.device_footprint_bytes(shape, self.npml, self.dtype, lossy=True)
+        if 8 * own <= self._memory_budget:
+            return True  # the headroom holds it; the query below costs 0.1 to 2 ms
         torch = _torch()
         free, total = torch.cuda.mem_get_info(self.device)
 
         def fits(free):
-            return self._second_psi_h_fits((self.Nx, self.Ny, self.Nz), self.npml, self.dtype,
-                                           self._memory_budget, free, total)
+            return self._second_psi_h_fits(shape, self.npml, self.dtype, self._memory_budget,
+                                           free, total)
 
         return fits(free) or fits(free + torch.cuda.memory_reserved(self.device)
                                   - torch.cuda.memory_allocated(self.device))

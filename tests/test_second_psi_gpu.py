@@ -40,6 +40,20 @@ def test_second_set_only_where_it_is_used(cuda, shape, npml, made):
     assert cuda.CUDAFDTD(shape, 1e-3, npml=npml, fused=False)._psi_hn is None
 
 
+def test_second_set_asks_for_room_on_a_small_device(cuda, monkeypatch):
+    """A grid above an eighth of the budget asks what is free."""
+    asked = []
+    monkeypatch.setattr(cuda.CUDAFDTD, "_second_psi_h_fits",
+                        staticmethod(lambda *a: asked.append(a)))
+    assert cuda.CUDAFDTD((192, 192, 192), 1e-3, npml=8)._psi_hn is not None and not asked
+    monkeypatch.setattr(cuda.CUDAFDTD, "device_memory_budget_bytes",
+                        staticmethod(lambda device: 4 * 10**9))
+    assert cuda.CUDAFDTD((192, 192, 192), 1e-3, npml=8)._psi_hn is None
+    shape, npml, dtype, budget, free, total = asked[0]
+    assert (shape, npml, dtype, budget) == ((192, 192, 192), 8, np.dtype("float32"), 4 * 10**9)
+    assert 0 < free <= total
+
+
 def test_slabs_have_no_second_set(cuda):
     for s in slabs.partition(384, 3, 8):
         g = cuda.CUDAFDTD((384, 192, 192), 1e-3, npml=8, slab=s)
@@ -55,7 +69,7 @@ def test_slabs_have_no_second_set(cuda):
 def test_step_in_place_vs_oracle(cuda, shape, npml, lossy, schedule, dtype, monkeypatch):
     from opencl_fdtd_solver_b200 import _capi as capi
 
-    monkeypatch.setattr(cuda.CUDAFDTD, "_second_psi_h_fits", lambda *a: False)
+    monkeypatch.setattr(cuda.CUDAFDTD, "_second_psi_h_pays", lambda self: False)
     nx, ny, nz = shape
     rng = np.random.default_rng(23)
     g = cuda.CUDAFDTD(shape, 1e-3, npml=npml, dtype=dtype)
