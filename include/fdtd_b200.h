@@ -146,10 +146,10 @@ int fdtd_step(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
  * every advanced ψ_H value written to psi_h_next (all six set, none aliasing
  * psi_h; may be NULL when npml == 0), and the caller swaps the two sets along
  * with E/E_next and H/H_next; ψ_E in place.  With ψ_H kept, a CTA can evaluate
- * H^{n+1/2} of a neighbour's CPML cell, so whole grids whose step exceeds the L2
- * (two million FP32 cells and more, rows a multiple of 16 bytes) take one march
- * over all cells instead of fdtd_step's interior and shell launches.  Same
- * results bit for bit. */
+ * H^{n+1/2} of a neighbour's CPML cell, so most whole grids whose step exceeds the
+ * L2 (two million FP32 cells and more, rows a multiple of 16 bytes) take one march
+ * over all cells instead of fdtd_step's interior and shell launches
+ * (fdtd_step_schedule tells).  Same results bit for bit. */
 int fdtd_step_swap(const fdtd_grid *g, const fdtd_fields *f, const fdtd_cpml *c,
                    const fdtd_source *src, int32_t nsrc,
                    const fdtd_plane_dft *planes, int32_t nplanes, void *stream);
@@ -268,7 +268,7 @@ int fdtd_n2f_workspace(const fdtd_n2f_face *faces, int32_t nfaces, int32_t nfreq
  * [nfreq][n_obs][6] for the tensor-core modes, complex128 for FDTD_N2F_FP64.
  * The tensor-core modes pack the currents into the workspace (256-byte
  * aligned; split-BF16 packs the sums and differences of the samples about each
- * face's middle), run one CTA per (128 directions, one or more faces, frequency)
+ * face's middle, and sums a direction again in float64 where they leave float32), run one CTA per (128 directions, one or more faces, frequency)
  * and reduce the faces; bounded waits set bit 1 of fdtd_device_status on timeout. */
 int fdtd_n2f_contract(const fdtd_n2f_face *faces, int32_t nfaces, int32_t cur_dtype,
                       const double *freqs, int32_t nfreq, const double *dirs, int32_t n_obs,

@@ -1,8 +1,10 @@
 // Fused Yee step for sm_100a: one pass over HBM for the interior of the grid.
 //
-// Schedules: a whole grid stepped with ψ_H double-buffered (fdtd_step_swap) and
-// too large for the L2 takes one march over every cell (yee_march.cu).  The
-// others (ψ_H in place, x-slabs, odd rows, small grids) run, on two streams:
+// Schedules (step_schedule): a whole grid stepped with ψ_H double-buffered
+// (fdtd_step_swap) and too large for the L2 takes one march over every cell
+// (yee_march.cu); grids that fit the L2, odd rows and lossy media two launches over
+// every cell (yee_shell.cu).  The others (large lossless grids with ψ_H in place,
+// x-slabs, the smallest grids) run, on two streams:
 //   side stream, forked from the caller's stream:
 //   1. k_shell_H   (yee_shell.cu): H^{n+1/2} on the CPML shell outside the box
 //                  B = [npml, N-npml)^3, psi_H in place, into H_next.
@@ -853,13 +855,13 @@ static cudaError_t launch_step_grid(const YeeArgs<T> &a, const SourceList &src,
 // for the shell kernels) hold two fifths of the rows, and, unless interior_pays or
 // interior_beats_grid, all that could have marched (a second ψ_H given).  The interior
 // march with shell kernels keeps the rest.  Measured per step, two launches / interior
-// march, in us: FP32 with a
-// source and a plane DFT 48³ 13.5 / 24.7, 64³ 16.4 / 25.3, 96³ 28.0 / 31.4; lossy FP32
-// 280x216x80 npml 6 110 / 158, 256³ npml 12 336 / 381, FP64 160³ npml 4 142 / 176, 384³
-// npml 16 1840 / 1993; lossless FP32 300x300x60 npml 20 133.0 / 163.8, 160x160x96 npml 12
-// 58.5 / 65.6, but 384³ FP64 npml 16 1733 / 1535 for a caller that steps in place.
-// The two launches win below the line too (40x36x48 14.3 / 27.3), but the bounded
-// waits of the interior march and its launch counts are tested on such a grid.
+// march, in us: FP32 with a z-plane DFT 48³ 9.8 / 22.6, 64³ 13.0 / 23.0, 96³ 22.6 / 29.1,
+// 128³ 50.0 / 51.8; lossy FP32 280x216x80 npml 6 110 / 157, 256³ npml 12 336 / 379, FP64 160³
+// npml 4 142 / 175, 384³ npml 16 1838 / 1989; lossless FP32 300x300x60 npml 20 130 / 164,
+// 160x160x96 npml 12 57.6 / 64.7, but 384³ FP64 npml 16 1737 / 1530 for a caller that steps
+// in place.  The two launches win below the line too (40x36x48 8.9 / 24.8, 44³ 9.3 / 22.7):
+// no measurement puts it at 100,000 cells, but the bounded waits of the interior march and
+// its launch counts are tested on a grid of 69,120.
 constexpr int64_t GRID_MIN_CELLS = 100000;
 
 // Interior H box B = [npml, N-npml)^3 (x on a slab: [pml_lo, nx - pml_hi -

@@ -75,9 +75,9 @@ inline double pml_fraction(int nx, int ny, int nz, int npml) {
 // The march takes grids whose step (15 arrays: six fields read, six written,
 // three coefficients) clearly exceeds the 126 MB L2.  Below, more threads beat
 // fewer bytes: the march's planes follow one another, about 1.7 us each.
-// Measured per step with a source and a plane DFT, march against one whole-grid H
-// and one E launch: FP32 64³ 20.6 / 16.4 us, 96³ 29.8 / 28.0, 128³ 64.4 / 59.7,
-// 160x160x96 69.1 / 69.8, 192³ 141.9 / 174.5; FP64 96³ 62.3 / 44.2, 128³ 85.5 / 95.9.
+// Measured per step with a z-plane DFT, march against one whole-grid H and one E
+// launch: FP32 64³ 18.4 / 13.0 us, 96³ 28.3 / 22.6, 128³ 55.4 / 50.0, 160³ 89.7 / 89.6,
+// 192³ 124.1 / 143.5; FP64 96³ 44.6 / 35.8, 112³ 62.2 / 58.2, 128³ 79.2 / 81.2.
 constexpr int64_t MARCH_MIN_BYTES = 140000000;
 template <typename T>
 inline bool march_size(int64_t cells) {
@@ -92,9 +92,11 @@ inline double tile_pad(int ny, int nz, int tk, int tj) {
 // Lossless grids that the march's tiles pad and whose z slabs are a tenth of the rows
 // at most stay with the interior march and its shell kernels, if the planes are few.
 // Per step in us, interior march / march / two whole-grid launches: FP32 72x224x328
-// npml 4 82.1 / 96.0 / 94.5, 200³ npml 4 126.8 / 142.7 / 139.7, 328x224x208 npml 8 234 /
-// 245 / 266, but 368x224x272 npml 4 345 / 316 / 370; FP64 48x292x104 npml 4 54.3 / 62.6 /
-// 54.9, 120x239x136 npml 4 115 / 127 / 129, but 355x136x52 npml 6 117.8 / 91.6 / 95.2.
+// npml 4 81.8 / 96.0 / 94.3, 200³ npml 4 127.8 / 140.8 / 139.1, 328x224x208 npml 8 232 /
+// 243 / 265, but 368x224x272 npml 4 344 / 316 / 369; FP64 48x292x104 npml 4 52.9 / 61.8 /
+// 55.0, 120x239x136 npml 4 114 / 126 / 128, but 355x136x52 npml 6 118.8 / 90.5 / 94.8.
+// (Just above the line of 1.05 the march can win: FP32 256x168x304 npml 6, padded by
+// 1.053, 206.8 / 200.4 / 221.5.)
 inline bool interior_pays(int nx, int nz, int npml, double pad) {
     return pad > 1.05 && nz >= 20 * npml && (nx <= 256 || pad > 1.2);
 }
@@ -125,13 +127,16 @@ inline bool interior_beats_grid(int nx, int ny, int nz, int npml) {
 // cells in fewer, longer threads, its padding is work, and the narrower tile streams
 // less well in FP32.  In ps per cell, f the CPML fraction, lossless FP32 grids below
 // 10 M cells take about pad (11 + 20 f), 1.45 times that in narrow tiles, against 18 +
-// 7 f; measured, march / whole-grid launches in us: 192³ npml 20 132 / 149, 160x160x96
-// npml 12 (narrow) 63.7 / 58.5, 280x216x80 npml 6 (narrow) 145.8 / 99.0, 240x48x280 npml
-// 10 97 / 72, 150x136x176 npml 10 82.2 / 74.7.  Above, the bytes count: 344x136x272 npml
-// 16 216 / 241, 398x160x336 npml 20 351 / 404.  FP64: 192³ npml 8 194.5 / 227.6,
-// 34x483x224 npml 13 172 / 158, 384³ npml 16 1365 / 1733.  Lossy (a deeper read per cell,
-// one stage less in the ring): 192³ npml 20 158 / 164, 256³ npml 12 327 / 336, but padded
-// 200³ npml 4 194.9 / 157.6 and FP64 192³ npml 8 268.5 / 240.6.
+// 7 f; measured, march / whole-grid launches in us: 192³ npml 20 132 / 148, 280x216x80 npml
+// 6 (narrow) 108 / 98, 240x48x280 npml 10 79 / 71, but 160x160x96 npml 12 (narrow) 53.1 /
+// 57.7 goes to the launches and 150x136x176 npml 10 82.4 / 74.0 to the march: chunks are
+// whole planes, and the estimate is good to a tenth.  Above, the bytes count: 344x136x272
+// npml 16 214 / 241, 398x160x336 npml 20 350 / 405.  FP64: 192³ npml 8 193 / 227,
+// 34x483x224 npml 13 170 / 156, 384³ npml 16 1366 / 1737.  Lossy (a deeper read per cell,
+// one stage less in the ring): 192³ npml 20 159 / 163, 256³ npml 12 326 / 336, but padded
+// 200³ npml 4 194 / 157 and FP64 192³ npml 8 (interior march) 300 / 240.
+// Of 1460 random grids of 0.4 M to 200 M cells with npml 3 to 20, 18 run more than 5 %
+// (one 17 %) slower by all these rules than by the interior march; their mean is 13 % faster.
 template <typename T>
 inline bool march_pays(int nx, int ny, int nz, int npml, bool lossy, bool narrow, double pad) {
     const int64_t cells = (int64_t)nx * ny * nz;

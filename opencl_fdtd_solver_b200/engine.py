@@ -12,10 +12,10 @@ Reference contract (``opencl_fdtd_solver/engine.py``):
 
 Design.  Torch tensors own every device buffer; the kernels are reached only
 through the C ABI of ``libfdtd_b200.so`` (``_capi.py``).  A step normally runs
-fused (``fdtd_step_swap``, fields and ψ_H double-buffered): source callbacks are executed *before* the
-launch, with ``t`` at the half step, and their ``add_source_*`` calls are
-recorded and applied in the kernel to ``E^n`` ahead of the E update, which is
-exactly the reference ordering (H^{n+½} never depends on the injection).  If a
+fused (``fdtd_step``, fields double-buffered; ``fdtd_step_swap``, ψ_H too, for grids that
+march): source callbacks are executed *before* the launch, with ``t`` at the half step,
+and their ``add_source_*`` calls are recorded and applied in the kernel to ``E^n`` ahead
+of the E update, which is exactly the reference ordering (H^{n+½} never depends on the injection).  If a
 source callback touches field state (any field property or view), the engine
 first materialises ``H^{n+½}`` with the split H kernel, applies the recorded
 injections, and finishes the step with the split E kernel — so arbitrary

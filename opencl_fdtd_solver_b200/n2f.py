@@ -64,6 +64,9 @@ def near2far_contract(faces, freqs, directions, mode="bf16x3", *, stream=None):
                  ``"fp64"`` (float64 direct sum, complex128 result).  Error against
                  the float64 sums, over their peak: ``"bf16x3"`` ≤ 1e-5 (about 5e-6
                  measured); ``"tf32"`` about 3e-4, outside the 1e-5 class.
+                 ``"bf16x3"`` sums up to four currents before it rounds them; a
+                 direction whose sums leave float32 (currents of 8.5e37 and more) is
+                 summed again in float64, which is slow.
     """
     if mode not in MODES:
         raise ValueError(f"mode must be one of {sorted(MODES)}, got {mode!r}")
